@@ -45,60 +45,100 @@ constexpr int D3_T = 256;
 
 // sim.rs:177: alpha += (alpha_target - alpha) * alpha_decay, each operation
 // rounded on its own (no fused multiply-add), as the reference computes it.
-__global__ void k_d3_alpha(D3State *s, double decay) {
-    s->alpha = __dadd_rn(s->alpha, __dmul_rn(__dsub_rn(s->alpha_target, s->alpha), decay));
+__device__ __forceinline__ double d3_cool(double alpha, double target, double decay) {
+    return __dadd_rn(alpha, __dmul_rn(__dsub_rn(target, alpha), decay));
 }
 
-__global__ void k_d3_end(D3State *s) { s->tick_no++; }
-
-// Projected records {x + vx, y + vy, 0, 1}: the link's state (link.rs
-// displaced) and collide's tree input (collide.rs prepare).
+// Projected records {x + vx, y + vy, degree, 1}: the link's state (link.rs
+// displaced). The degree rides along so that the link pass reads a neighbour in
+// one 16-byte load. Thread 0 also advances the cooling schedule and the tick
+// count, which nothing else in this kernel reads; the tick's later kernels key
+// their jiggles on tick_no - 1.
 __global__ void k_d3_project(uint32_t n, const float4 *__restrict__ p, const float2 *__restrict__ v,
-                             float4 *__restrict__ pp) {
+                             const uint32_t *__restrict__ rp, float4 *__restrict__ pp, D3State *s, double decay) {
     const uint32_t i = blockIdx.x * D3_T + threadIdx.x;
+    if (i == 0) {
+        s->alpha = d3_cool(s->alpha, s->alpha_target, decay);
+        s->tick_no++;
+    }
     if (i >= n) return;
     const float4 a = p[i];
     const float2 b = v[i];
-    pp[i] = make_float4(a.x + b.x, a.y + b.y, 0.f, 1.f);
+    pp[i] = make_float4(a.x + b.x, a.y + b.y, (float)(rp[i + 1] - rp[i]), 1.f);
 }
 
-// Node v's share of its simple edge to u (link.rs force + share).
-__device__ __forceinline__ void d3_link_term(const D3Params &P, uint32_t v, uint32_t u, float s, float alpha,
-                                             uint32_t tick, const float4 *__restrict__ pp,
-                                             const uint32_t *__restrict__ rp, float &ax, float &ay) {
-    const uint32_t lo = min(u, v), hi = max(u, v);
-    const float4 a = pp[hi], b = pp[lo];
-    float dx = a.x - b.x, dy = a.y - b.y;
-    if (dx == 0.f) dx = (float)jiggle(P.seed, tick, 0, lo, hi);
-    if (dy == 0.f) dy = (float)jiggle(P.seed, tick, 1, lo, hi);
+// One directed CSR entry of the link pass, laid out once per session: the
+// neighbour, the rest length and strength of its edge, and this row's signed
+// share of the correction (link.rs force and share: -bias for the edge's higher
+// node, 1 - bias for the lower, bias = the lower node's part of the degrees).
+// Per tick that leaves a node one square root and one division an entry; with
+// the degrees, the rest length and the share worked out every tick (two divisions
+// and two random reads of row offsets an entry more) the pass took 112 us at 1M
+// nodes and 3.1M entries, with the table 67 us.
+struct D3Link {
+    uint32_t u;
+    float dist, str, share;
+};
+
+__global__ void k_d3_link_table(D3Params P, uint32_t n, const uint32_t *__restrict__ rp,
+                                const uint32_t *__restrict__ col, const float *__restrict__ wt, uint32_t ne,
+                                D3Link *__restrict__ lk) {
+    const uint32_t e = blockIdx.x * D3_T + threadIdx.x;
+    if (e >= ne) return;
+    uint32_t lo = 0, hi = n;  // the row of entry e: the last r with rp[r] <= e
+    while (hi - lo > 1) {
+        const uint32_t mid = lo + (hi - lo) / 2;
+        if (rp[mid] <= e) lo = mid;
+        else hi = mid;
+    }
+    const uint32_t v = lo, u = col[e];
+    const float s = wt[e];
+    const uint32_t a = min(u, v), b = max(u, v);
+    const float dlo = (float)(rp[a + 1] - rp[a]), dhi = (float)(rp[b + 1] - rp[b]);
+    const float bias = dlo / (dlo + dhi);
+    lk[e] = D3Link{u, P.link_distance / fmaxf(0.4f, s), fminf(0.7f, P.link_strength_scale * s),
+                   v == b ? -bias : 1.f - bias};
+}
+
+// Node v's share of one simple edge (link.rs force + share); me = pp[v].
+__device__ __forceinline__ void d3_link_term(const D3Params &P, uint32_t v, const float4 &me, const D3Link &k,
+                                             float alpha, uint32_t tick, const float4 *__restrict__ pp, float &ax,
+                                             float &ay) {
+    const float4 o = pp[k.u];
+    const bool high = v > k.u;  // the displacement runs from the lower node to the higher
+    float dx = high ? me.x - o.x : o.x - me.x, dy = high ? me.y - o.y : o.y - me.y;
+    if (dx == 0.f || dy == 0.f) {
+        const uint32_t lo = min(k.u, v), hi = max(k.u, v);
+        if (dx == 0.f) dx = (float)jiggle(P.seed, tick, 0, lo, hi);
+        if (dy == 0.f) dy = (float)jiggle(P.seed, tick, 1, lo, hi);
+    }
     const float l = sqrtf(dx * dx + dy * dy);
     if (l == 0.f) return;
-    const float dist = P.link_distance / fmaxf(0.4f, s);
-    const float str = fminf(0.7f, P.link_strength_scale * s);
-    const float dlo = (float)(rp[lo + 1] - rp[lo]), dhi = (float)(rp[hi + 1] - rp[hi]);
-    const float bias = dlo / (dlo + dhi);
-    const float factor = (l - dist) / l * alpha * str;
-    if (v == hi) {
-        ax -= dx * factor * bias;
-        ay -= dy * factor * bias;
-    } else {
-        ax += dx * factor * (1.f - bias);
-        ay += dy * factor * (1.f - bias);
-    }
+    const float factor = (l - k.dist) / l * alpha * k.str;
+    ax += dx * factor * k.share;
+    ay += dy * factor * k.share;
+}
+
+__device__ __forceinline__ D3Link d3_link_load(const D3Link *__restrict__ lk, uint32_t e) {
+    const uint4 q = __ldg((const uint4 *)lk + e);
+    return D3Link{q.x, __uint_as_float(q.y), __uint_as_float(q.z), __uint_as_float(q.w)};
 }
 
 // Heavy rows: one warp per SEG-entry segment, summed by a fixed butterfly.
 __global__ void __launch_bounds__(D3_T)
 k_d3_link_seg(D3Params P, uint32_t nseg, const D3State *st, const float4 *__restrict__ pp,
-              const uint32_t *__restrict__ rp, const uint32_t *__restrict__ col, const float *__restrict__ wt,
-              const uint32_t *__restrict__ seg_row, const uint32_t *__restrict__ seg_first, float2 *__restrict__ seg_out) {
+              const uint32_t *__restrict__ rp, const D3Link *__restrict__ lk, const uint32_t *__restrict__ seg_row,
+              const uint32_t *__restrict__ seg_first, float2 *__restrict__ seg_out) {
     const uint32_t sg = (blockIdx.x * D3_T + threadIdx.x) / GR_WARP, lane = threadIdx.x % GR_WARP;
     if (sg >= nseg) return;
     const uint32_t row = seg_row[sg];
     const uint32_t e0 = rp[row] + (sg - seg_first[row]) * SEG, e1 = min(e0 + SEG, rp[row + 1]);
     const float alpha = (float)st->alpha;
     float ax = 0.f, ay = 0.f;
-    for (uint32_t e = e0 + lane; e < e1; e += GR_WARP) d3_link_term(P, row, col[e], wt[e], alpha, st->tick_no, pp, rp, ax, ay);
+    const uint32_t tick = st->tick_no - 1u;
+    const float4 me = pp[row];
+    for (uint32_t e = e0 + lane; e < e1; e += GR_WARP)
+        d3_link_term(P, row, me, d3_link_load(lk, e), alpha, tick, pp, ax, ay);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         ax += __shfl_xor_sync(GR_FULL, ax, o);
@@ -111,15 +151,17 @@ k_d3_link_seg(D3Params P, uint32_t nseg, const D3State *st, const float4 *__rest
 // segments in order) onto its own velocity. Reads only the projected records.
 __global__ void __launch_bounds__(D3_T)
 k_d3_link(D3Params P, const D3State *st, const float4 *__restrict__ pp, const uint32_t *__restrict__ rp,
-          const uint32_t *__restrict__ col, const float *__restrict__ wt, const uint32_t *__restrict__ seg_first,
-          const float2 *__restrict__ seg_out, float2 *__restrict__ v) {
+          const D3Link *__restrict__ lk, const uint32_t *__restrict__ seg_first, const float2 *__restrict__ seg_out,
+          float2 *__restrict__ v) {
     const uint32_t i = blockIdx.x * D3_T + threadIdx.x;
     if (i >= P.n) return;
     const float alpha = (float)st->alpha;
     const uint32_t e0 = rp[i], e1 = rp[i + 1];
     float ax = 0.f, ay = 0.f;
     if (seg_first == nullptr || e1 - e0 <= LIGHT_MAX) {
-        for (uint32_t e = e0; e < e1; e++) d3_link_term(P, i, col[e], wt[e], alpha, st->tick_no, pp, rp, ax, ay);
+        const uint32_t tick = st->tick_no - 1u;
+        const float4 me = pp[i];
+        for (uint32_t e = e0; e < e1; e++) d3_link_term(P, i, me, d3_link_load(lk, e), alpha, tick, pp, ax, ay);
     } else {
         const uint32_t s0 = seg_first[i], ns = (e1 - e0 + SEG - 1) / SEG;
         for (uint32_t s = s0; s < s0 + ns; s++) {
@@ -165,7 +207,7 @@ k_d3_charge(D3Params P, const D3State *st, const DevState *ts, Cells cells, cons
             const uint32_t *__restrict__ sorig, float2 *__restrict__ v) {
     const uint32_t p = blockIdx.x * D3_T + threadIdx.x;
     if (p >= P.n) return;
-    const uint32_t ncells = ts->n_cells, tick = st->tick_no;
+    const uint32_t ncells = ts->n_cells, tick = st->tick_no - 1u;
     const float ca = P.charge * (float)st->alpha;
     const float4 me = sp[p];
     const uint32_t oi = sorig[p];
@@ -209,83 +251,221 @@ k_d3_charge(D3Params P, const D3State *st, const DevState *ts, Cells cells, cons
     v[oi] = w;
 }
 
-// center.js: every position shifted by the mean (FP64, from the bounds pass
-// over the same positions: the many-body tree's, or the mesh's) times the
-// centering strength.
-__global__ void k_d3_center(uint32_t n, float strength, const double *mean, float4 *__restrict__ p) {
-    const uint32_t i = blockIdx.x * D3_T + threadIdx.x;
-    if (i >= n) return;
-    const float sx = (float)(mean[0] * (double)strength), sy = (float)(mean[1] * (double)strength);
-    float4 a = p[i];
-    a.x -= sx;
-    a.y -= sy;
-    p[i] = a;
+// ---- collide: every other point within reach = 2 r of the projected position
+// pushed apart by half the overlap (collide.rs). The points are sorted by the
+// Morton key the quadtree would use, and cut into the dyadic cells of its root
+// square at the deepest level whose cells are still at least `reach` wide; a
+// node's partners then lie in the 3 x 3 cells around its own, each a run of
+// sorted points. Taking the runs in sorted order adds the same terms in the same
+// order as a walk of the quadtree's leaves, bit for bit. That quadtree and its
+// walk stood here before: at 1M nodes the leaf pass, the radix tree, the scan,
+// the cell writer and the walk took 595 us of the tick, the gather and the scan
+// of the cells take 290 us.
+//
+// The runs are found in a table of one entry a cell, as many entries as nodes or
+// more. A drawing whose box needs a deeper level than the table holds
+// (a few far outliers) looks its cells up by bisection inside the table's
+// coarser ones, or, one level too deep, takes the coarser cells as they are.
+// However crowded the cells are, the points looked at stay within a small
+// multiple of the pairs in reach, because a cell's points pair up among
+// themselves.
+
+struct D3Grid {
+    int level, table_level;  // of the cells taken, and of the table's (<= level)
+    uint32_t ticket, pad;
+};
+
+// Table levels for n nodes: 4^level >= n entries, at least 4^6.
+__host__ __device__ inline int d3_table_level(uint32_t n) {
+    int l = 6;
+    while (l < 14 && (1ull << (2 * l)) < n) l++;
+    return l;
 }
 
-// collide.js over the tree of projected positions: leaves take every other
-// point within 2 r, internal cells whose square lies beyond reach are skipped
-// (with a margin, so rounding never skips a point that counts).
+// center.js: every position shifted by the mean (FP64, from the bounds pass over
+// the same positions: the many-body tree's, or the mesh's) times the centering
+// strength; then the projected records collide reads (collide.rs prepare), and,
+// in the last block, their root square and the cells' levels. Also zeroes the
+// sort's counters and the cell table. A non-finite projected position ends the
+// tick. `widest` is more than any pair in reach is apart on one axis.
+__global__ void __launch_bounds__(BND_THREADS)
+k_d3_center(uint32_t n, float strength, const double *mean, float4 *__restrict__ p, const float2 *__restrict__ v,
+            float4 *__restrict__ pp, DevState *ts, double widest, int table_level, double *__restrict__ part,
+            D3Grid *grid, uint2 *__restrict__ table, ZeroWords zw) {
+    __shared__ float s_m[4][BND_THREADS / GR_WARP];
+    __shared__ double s_d[4][BND_THREADS / GR_WARP];
+    __shared__ bool s_last;
+    if (blockIdx.x == 0) zw.clear();
+    const float sx = (float)(mean[0] * (double)strength), sy = (float)(mean[1] * (double)strength);
+    float m[4] = {INFINITY, INFINITY, INFINITY, INFINITY};  // min x, min y, -max x, -max y
+    bool bad = false;
+    const uint32_t stride = gridDim.x * BND_THREADS, first = blockIdx.x * BND_THREADS + threadIdx.x;
+    for (uint32_t i = first; i < n; i += stride) {
+        float4 a = p[i];
+        const float2 b = v[i];
+        a.x -= sx;
+        a.y -= sy;
+        p[i] = a;
+        const float x = a.x + b.x, y = a.y + b.y;
+        pp[i] = make_float4(x, y, 0.f, 1.f);
+        bad = bad || !(isfinite(x) && isfinite(y));
+        m[0] = fminf(m[0], x);
+        m[1] = fminf(m[1], y);
+        m[2] = fminf(m[2], -x);
+        m[3] = fminf(m[3], -y);
+    }
+    for (uint32_t i = first; i < (1u << (2 * table_level)); i += stride) table[i] = make_uint2(0u, 0u);
+    if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(&ts->error, (uint32_t)ERR_NONFINITE);
+    const int lane = threadIdx.x % GR_WARP, w = threadIdx.x / GR_WARP;
+#pragma unroll
+    for (int a = 0; a < 4; a++) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m[a] = fminf(m[a], __shfl_xor_sync(GR_FULL, m[a], o));
+        if (lane == 0) s_m[a][w] = m[a];
+    }
+    __syncthreads();
+    if (threadIdx.x < 4) {
+        float l = INFINITY;
+        for (int k = 0; k < BND_THREADS / GR_WARP; k++) l = fminf(l, s_m[threadIdx.x][k]);
+        part[(size_t)blockIdx.x * 4 + threadIdx.x] = l;
+    }
+    if (!last_block_done(&grid->ticket, &s_last)) return;
+    double d[4] = {INFINITY, INFINITY, INFINITY, INFINITY};
+    for (uint32_t b = threadIdx.x; b < gridDim.x; b += BND_THREADS)
+#pragma unroll
+        for (int a = 0; a < 4; a++) d[a] = fmin(d[a], __ldcg(part + (size_t)b * 4 + a));
+#pragma unroll
+    for (int a = 0; a < 4; a++) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) d[a] = fmin(d[a], __shfl_xor_sync(GR_FULL, d[a], o));
+        if (lane == 0) s_d[a][w] = d[a];
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int a = 0; a < 4; a++)
+        for (int k = 0; k < BND_THREADS / GR_WARP; k++) d[a] = fmin(d[a], s_d[a][k]);
+    const double mn[2] = {d[0], d[1]}, mx[2] = {-d[2], -d[3]};
+    bool ok = true;
+    const double z = root_square<2>(mn, mx, ts->root0, ok);
+    if (!ok) atomicOr(&ts->error, (uint32_t)ERR_BOUNDS);
+    ts->root_w = z;
+    if (ts->error) ts->converged = 1;
+    // at level 1 the 3 x 3 cells are the whole square, however wide the reach
+    int level = 1;
+    for (double side = z * 0.25; level < 31 && side >= widest; side *= 0.5) level++;
+    if (level == table_level + 1) level = table_level;
+    grid->level = level;
+    grid->table_level = min(level, table_level);
+}
+
+// The sorted points' records (z: the node's id), and each occupied cell's first
+// and one-past-last point in the table.
 __global__ void __launch_bounds__(D3_T)
-k_d3_collide(D3Params P, const D3State *st, const DevState *ts, Cells cells, const float4 *__restrict__ sp,
-             const uint32_t *__restrict__ sorig, float2 *__restrict__ v) {
+k_d3_cells(uint32_t n, const DevState *ts, const D3Grid *grid, const float4 *__restrict__ pp,
+           const uint64_t *__restrict__ keys, const uint32_t *__restrict__ vals, float4 *__restrict__ sp,
+           uint2 *__restrict__ table) {
+    gr_pdl_enter();
+    const uint32_t q = blockIdx.x * D3_T + threadIdx.x;
+    if (q >= n || ts->converged) return;
+    const int shift = 64 - 2 * grid->table_level;
+    const uint64_t k = keys[q] >> shift;
+    const uint32_t i = vals[q];
+    float4 a = pp[i];
+    a.z = __uint_as_float(i);
+    sp[q] = a;
+    if (q == 0 || (keys[q - 1] >> shift) != k) table[k].x = q;
+    if (q + 1 == n || (keys[q + 1] >> shift) != k) table[k].y = q + 1;
+}
+
+// The first of the sorted points [lo, hi) whose key is at least k.
+__device__ __forceinline__ uint32_t d3_bisect(const uint64_t *__restrict__ keys, uint32_t lo, uint32_t hi, uint64_t k) {
+    while (lo < hi) {
+        const uint32_t mid = lo + (hi - lo) / 2;
+        if (__ldg(&keys[mid]) < k) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo;
+}
+
+// Collide, one thread per node in sorted order, and the tick's tail for that
+// node (simulation.js: v *= velocityDecay, x += v).
+__global__ void __launch_bounds__(D3_T)
+k_d3_collide(D3Params P, const D3State *st, const DevState *ts, const D3Grid *grid, const uint64_t *__restrict__ keys,
+             const float4 *__restrict__ sp, const uint2 *__restrict__ table, float4 *__restrict__ pos,
+             float2 *__restrict__ v) {
+    gr_pdl_enter();
     const uint32_t p = blockIdx.x * D3_T + threadIdx.x;
-    if (p >= P.n) return;
-    const uint32_t ncells = ts->n_cells, tick = st->tick_no;
+    if (p >= P.n || ts->converged) return;
+    const uint32_t tick = st->tick_no - 1u;
+    const int level = grid->level, deeper = 2 * (level - grid->table_level), shift = 64 - 2 * level;
     const float4 q = sp[p];
-    const uint32_t oi = sorig[p];
-    const float prune = P.reach * 1.0001f;
-    float ax = 0.f, ay = 0.f;
-    uint32_t k = 0;
-    while (k < ncells) {
-        const float4 B = cell_b<2>(cells, k);
-        const int32_t sk = __float_as_int(B.z);
-        if (sk < 0) {
-            const uint32_t start = __float_as_uint(B.w), cnt = (uint32_t)(-sk);
-            for (uint32_t j = start; j < start + cnt; j++) {
-                if (j == p) continue;
-                const float4 o = __ldg(&sp[j]);
-                float dx = q.x - o.x, dy = q.y - o.y;
-                float l = dx * dx + dy * dy;
-                if (l >= P.reach2) continue;
-                const uint32_t oj = __ldg(&sorig[j]);
-                if (dx == 0.f) {
-                    dx = (float)jiggle(P.seed, tick, 4, oi, oj);
-                    l += dx * dx;
-                }
-                if (dy == 0.f) {
-                    dy = (float)jiggle(P.seed, tick, 5, oi, oj);
-                    l += dy * dy;
-                }
-                const float dist = sqrtf(l);
-                const float push = (P.reach - dist) / dist * 0.5f;
-                ax += dx * push;
-                ay += dy * push;
-            }
-            k++;
-        } else {
-            const float4 b = __ldg(&cells.bounds[k]);
-            const bool out = b.x > q.x + prune || b.z < q.x - prune || b.y > q.y + prune || b.w < q.y - prune;
-            k = out ? max((uint32_t)sk, k + 1) : k + 1;
+    const uint32_t oi = __float_as_uint(q.z);
+    // the cell's coordinates from its Morton index, and its neighbours' runs
+    const uint64_t cell = keys[p] >> shift;
+    const uint32_t cx = compact2(cell), cy = compact2(cell >> 1), top = (1u << level) - 1u;
+    uint32_t lo[9], hi[9];
+#pragma unroll
+    for (int r = 0; r < 9; r++) {
+        const uint32_t x = cx + (uint32_t)(r % 3) - 1u, y = cy + (uint32_t)(r / 3) - 1u;
+        lo[r] = 0xffffffffu;  // no points: sorts last
+        hi[r] = 0u;
+        if (x > top || y > top || !(P.reach2 > 0.f)) continue;
+        const uint64_t c = spread2(x) | (spread2(y) << 1);
+        uint2 e = __ldg(&table[c >> deeper]);
+        if (deeper && e.x < e.y) {
+            e.x = d3_bisect(keys, e.x, e.y, c << shift);
+            e.y = ((c + 1) << shift) == 0ull ? e.y : d3_bisect(keys, e.x, e.y, (c + 1) << shift);
+        }
+        if (e.x < e.y) {
+            lo[r] = e.x;
+            hi[r] = e.y;
         }
     }
+#pragma unroll
+    for (int a = 1; a < 9; a++)  // the runs in sorted order (an insertion network)
+#pragma unroll
+        for (int b = a; b > 0; b--) {
+            const bool swap = lo[b] < lo[b - 1];
+            const uint32_t l0 = swap ? lo[b] : lo[b - 1], l1 = swap ? lo[b - 1] : lo[b];
+            const uint32_t h0 = swap ? hi[b] : hi[b - 1], h1 = swap ? hi[b - 1] : hi[b];
+            lo[b - 1] = l0;
+            lo[b] = l1;
+            hi[b - 1] = h0;
+            hi[b] = h1;
+        }
+    float ax = 0.f, ay = 0.f;
+#pragma unroll
+    for (int r = 0; r < 9; r++)
+        for (uint32_t j = lo[r]; j < hi[r]; j++) {
+            if (j == p) continue;
+            const float4 o = __ldg(&sp[j]);
+            float dx = q.x - o.x, dy = q.y - o.y;
+            float l = dx * dx + dy * dy;
+            if (l >= P.reach2) continue;
+            const uint32_t oj = __float_as_uint(o.z);
+            if (dx == 0.f) {
+                dx = (float)jiggle(P.seed, tick, 4, oi, oj);
+                l += dx * dx;
+            }
+            if (dy == 0.f) {
+                dy = (float)jiggle(P.seed, tick, 5, oi, oj);
+                l += dy * dy;
+            }
+            const float dist = sqrtf(l);
+            const float push = (P.reach - dist) / dist * 0.5f;
+            ax += dx * push;
+            ay += dy * push;
+        }
     float2 w = v[oi];
     w.x += ax;
     w.y += ay;
-    v[oi] = w;
-}
-
-// simulation.js tick tail: v *= velocityDecay, x += v.
-__global__ void k_d3_integrate(uint32_t n, float decay, float4 *__restrict__ p, float2 *__restrict__ v) {
-    const uint32_t i = blockIdx.x * D3_T + threadIdx.x;
-    if (i >= n) return;
-    float2 w = v[i];
-    w.x *= decay;
-    w.y *= decay;
-    float4 a = p[i];
+    w.x *= P.velocity_decay;
+    w.y *= P.velocity_decay;
+    float4 a = pos[oi];
     a.x += w.x;
     a.y += w.y;
-    v[i] = w;
-    p[i] = a;
+    v[oi] = w;
+    pos[oi] = a;
 }
 
 }  // namespace gr

@@ -2400,16 +2400,24 @@ int gr_stress(uint32_t n, uint64_t m, const uint32_t *source, const uint32_t *ta
 //
 // A d3-force Barnes-Hut session (d3force.cuh) over an internal FA2 handle that
 // holds the simple graph (CSR, edge strengths as weights, heavy-row segments),
-// the stream and the tree buffers; every tick is one captured CUDA graph that
-// builds the tree twice (positions for many-body, projected positions for
+// the stream and the tree buffers; every tick is one captured CUDA graph (the
+// tree of the positions for many-body, the sorted projected positions for
 // collide).
+
+constexpr uint32_t D3_CENTER_BLOCKS = 4 * 148;  // at most, of the pass that also takes the projected box
 
 struct gr_force_session {
     gr_fa2 *t = nullptr;
     uint32_t n = 0;
     gr_force_params prm{};
     D3Params P{};
-    float4 *p4 = nullptr, *pp4 = nullptr, *bounds = nullptr;
+    float4 *p4 = nullptr, *pp4 = nullptr;
+    D3Link *lk = nullptr;         // the link pass's CSR entries
+    D3Grid *grid = nullptr;       // collide's cells: their levels, the table of their runs, the box's block records
+    uint2 *table = nullptr;
+    double *box_part = nullptr;
+    int table_level = 0;
+    double widest = 0.0;          // more than any pair in reach is apart on one axis
     float2 *vel = nullptr, *seg_out = nullptr;
     D3State *ds = nullptr;
     cudaGraph_t graph = nullptr;
@@ -2496,32 +2504,33 @@ void d3_enqueue(gr_force_session *S) {
     gr_fa2 *t = S->t;
     cudaStream_t s = t->stream;
     const uint32_t n = S->n, g = div_up(n, D3_T);
-    k_d3_alpha<<<1, 1, 0, s>>>(S->ds, S->prm.alpha_decay);
-    k_d3_project<<<g, D3_T, 0, s>>>(n, S->p4, S->vel, S->pp4);
+    k_d3_project<<<g, D3_T, 0, s>>>(n, S->p4, S->vel, t->rp, S->pp4, S->ds, S->prm.alpha_decay);
     if (t->nseg)
         k_d3_link_seg<<<div_up((uint64_t)t->nseg * GR_WARP, D3_T), D3_T, 0, s>>>(
-            S->P, t->nseg, S->ds, S->pp4, t->rp, t->col, t->wt, t->seg_row, t->seg_first, S->seg_out);
-    k_d3_link<<<g, D3_T, 0, s>>>(S->P, S->ds, S->pp4, t->rp, t->col, t->wt, t->nseg ? t->seg_first : nullptr,
-                                 S->seg_out, S->vel);
+            S->P, t->nseg, S->ds, S->pp4, t->rp, S->lk, t->seg_row, t->seg_first, S->seg_out);
+    k_d3_link<<<g, D3_T, 0, s>>>(S->P, S->ds, S->pp4, t->rp, S->lk, t->nseg ? t->seg_first : nullptr, S->seg_out,
+                                 S->vel);
+    const double *mean;
     if (S->mesh) {  // many-body on the particle mesh
         pm_enqueue(S);
-        k_d3_center<<<g, D3_T, 0, s>>>(n, (float)S->prm.center_strength, S->pm->mean, S->p4);
+        mean = S->pm->mean;
     } else {  // many-body: the tree of the positions
         t->pos = S->p4;
         enqueue_tick<2>(t, false, PH_TREE);
         k_d3_charge<<<g, D3_T, 0, s>>>(S->P, S->ds, t->st, t->cells, t->sp, t->sorig, S->vel);
-        k_d3_center<<<g, D3_T, 0, s>>>(n, (float)S->prm.center_strength, t->st->mean, S->p4);
+        mean = t->st->mean;
     }
-    k_d3_project<<<g, D3_T, 0, s>>>(n, S->p4, S->vel, S->pp4);
-    t->pos = S->pp4;  // collide: the tree of the projected positions, with cell squares
-    t->cells.bounds = S->bounds;
-    enqueue_tick<2>(t, false, PH_TREE);
-    Cells cb = t->cells;
-    t->cells.bounds = nullptr;
+    ZeroWords zw;
+    zw.add(t->sorter.os_ghist, RadixSorter::ghist_words());
+    const uint32_t cb = std::min(g, D3_CENTER_BLOCKS);
+    k_d3_center<<<cb, BND_THREADS, 0, s>>>(n, (float)S->prm.center_strength, mean, S->p4, S->vel, S->pp4, t->st,
+                                           S->widest, S->table_level, S->box_part, S->grid, S->table, zw);
+    t->pos = S->pp4;  // the tree is done with the handle's key and sorted-point buffers
+    keys_sort_fast<2>(t, s);
     t->pos = S->p4;
-    k_d3_collide<<<g, D3_T, 0, s>>>(S->P, S->ds, t->st, cb, t->sp, t->sorig, S->vel);
-    k_d3_integrate<<<g, D3_T, 0, s>>>(n, (float)S->prm.velocity_decay, S->p4, S->vel);
-    k_d3_end<<<1, 1, 0, s>>>(S->ds);
+    gr_launch(t->pdl, k_d3_cells, g, D3_T, 0, s, n, t->st, S->grid, S->pp4, t->keys, t->vals, t->sp, S->table);
+    gr_launch(t->pdl, k_d3_collide, g, D3_T, 0, s, S->P, S->ds, t->st, S->grid, t->keys, t->sp, S->table, S->p4,
+              S->vel);
 }
 
 int d3_build_graph(gr_force_session *S) {
@@ -2611,8 +2620,18 @@ int gr_force_session_create(gr_force_session **out, uint32_t n, uint64_t m, cons
     P.velocity_decay = (float)prm.velocity_decay;
     P.alpha_decay = prm.alpha_decay;
     cudaError_t e;
-    if ((e = t->alloc(&S->p4, n)) || (e = t->alloc(&S->pp4, n)) || (e = t->alloc(&S->bounds, 2 * (size_t)n)) ||
-        (e = t->alloc(&S->vel, n)) || (e = t->alloc(&S->seg_out, std::max<uint32_t>(t->nseg, 1))) ||
+    const uint32_t ne = 2 * (uint32_t)t->m;
+    S->table_level = d3_table_level(n);
+    {
+        // the largest FP32 offset whose square stays below reach^2, and half an ulp
+        // (what rounding the offset itself can hide)
+        float d = std::sqrt(P.reach2);
+        while (d > 0.f && std::isfinite(P.reach2) && !(d * d < P.reach2)) d = std::nextafterf(d, 0.f);
+        S->widest = (double)d + 0.5 * ((double)std::nextafterf(d, INFINITY) - (double)d);
+    }
+    if ((e = t->alloc(&S->p4, n)) || (e = t->alloc(&S->pp4, n)) || (e = t->alloc(&S->lk, ne)) ||
+        (e = t->alloc(&S->grid, 1)) || (e = t->alloc(&S->box_part, 4 * (size_t)D3_CENTER_BLOCKS)) ||
+        (e = t->alloc(&S->table, (size_t)1 << (2 * S->table_level))) || (e = t->alloc(&S->vel, n)) || (e = t->alloc(&S->seg_out, std::max<uint32_t>(t->nseg, 1))) ||
         (e = t->alloc(&S->ds, 1))) {
         delete S;
         return set_err(GR_ALLOC_FAILED, cudaGetErrorString(e));
@@ -2633,6 +2652,8 @@ int gr_force_session_create(gr_force_session **out, uint32_t n, uint64_t m, cons
     }
     D3State d0{prm.initial_alpha, 0.0, 0u, 0u};
     cudaStream_t s = t->stream;
+    CU(cudaMemsetAsync(S->grid, 0, sizeof(D3Grid), s));
+    if (ne) k_d3_link_table<<<div_up(ne, D3_T), D3_T, 0, s>>>(S->P, n, t->rp, t->col, t->wt, ne, S->lk);
     if (n) {
         CU(cudaMemcpyAsync(S->p4, host.data(), (size_t)n * sizeof(float4), cudaMemcpyHostToDevice, s));
         CU(cudaMemsetAsync(S->vel, 0, (size_t)n * sizeof(float2), s));

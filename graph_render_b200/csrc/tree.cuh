@@ -46,6 +46,16 @@ __device__ __forceinline__ uint64_t spread2(uint64_t x) {  // 32 bits -> even bi
     return x;
 }
 
+// The even bits of x, packed (spread2's inverse).
+__device__ __forceinline__ uint32_t compact2(uint64_t x) {
+    x &= 0x5555555555555555ull;
+    x = (x | (x >> 1)) & 0x3333333333333333ull;
+    x = (x | (x >> 2)) & 0x0f0f0f0f0f0f0f0full;
+    x = (x | (x >> 4)) & 0x00ff00ff00ff00ffull;
+    x = (x | (x >> 8)) & 0x0000ffff0000ffffull;
+    return (uint32_t)((x | (x >> 16)) & 0xffffffffull);
+}
+
 __device__ __forceinline__ uint64_t spread3(uint64_t x) {  // 21 bits -> every third bit
     x &= 0x1fffffull;
     x = (x | (x << 32)) & 0x001f00000000ffffull;
@@ -975,7 +985,6 @@ template <int D> struct CellF { static constexpr uint32_t F = D == 3 ? 3 : 1; };
 struct Cells {
     float4 *rec;     // 2D: A of cell k at rec[k]; 3D: cell k's A, B, C at rec[3k ..]
     float4 *rec_b;   // 2D: B of cell k at rec_b[k]; 3D: unused
-    float4 *bounds;  // nullable: each cell's square {x0, y0, x1, y1} (2D), for range pruning
 };
 
 template <int D>
@@ -997,18 +1006,7 @@ __host__ __device__ inline Cells cells_view(float4 *buf, uint32_t cap, int dim) 
     Cells c;
     c.rec = buf;
     c.rec_b = dim == 3 ? nullptr : buf + cap;
-    c.bounds = nullptr;
     return c;
-}
-
-// The square of the level-`level` cell holding point p: the root corner plus
-// floor((p - corner) / w) sides, exact in FP64 (w is a power of two times the
-// root side). Rounded to FP32 it still contains every point of the cell.
-__device__ __forceinline__ void write_bounds(Cells c, uint32_t idx, const float4 &p, int level, const DevState *st) {
-    const double w = ldexp(st->root_w, -level);
-    const double bx = st->root0[0] + floor(((double)p.x - st->root0[0]) / w) * w;
-    const double by = st->root0[1] + floor(((double)p.y - st->root0[1]) / w) * w;
-    c.bounds[idx] = make_float4((float)bx, (float)by, (float)(bx + w), (float)(by + w));
 }
 
 template <int D>
@@ -1077,7 +1075,6 @@ __global__ void k_assign_cells(const DevState *st, BinTree t, uint32_t n_slots, 
         // the parent's record only for coincident points (one leaf alone is the root)
         const int level = nu == 1 ? 0 : coinc ? t.rec[t.leaf_parent[s]].w / D + 1 : L;
         write_cell<D>(cells, idx, body, level, rw, -(int32_t)(a1 - a0), a0, a1 - a0 == 1 ? &one : nullptr);
-        if (D == 2 && cells.bounds) write_bounds(cells, idx, one, level, st);
         leaf_pre[s] = idx;
         return;
     }
@@ -1095,7 +1092,6 @@ __global__ void k_assign_cells(const DevState *st, BinTree t, uint32_t n_slots, 
     const uint32_t a0 = leaf_start[f];
     pre.nu = nu;
     write_cell<D>(cells, idx, range_body(prefix_at<D>(pre, f), prefix_at<D>(pre, end)), lv, rw, (int32_t)skip, a0);
-    if (D == 2 && cells.bounds) write_bounds(cells, idx, sp[a0], lv, st);
     if (t.cell_of) t.cell_of[i] = idx;
 }
 
