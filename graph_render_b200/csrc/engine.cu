@@ -1014,6 +1014,28 @@ static int tick_impl(gr_fa2 *h, uint32_t ticks, float *dev_out, uint32_t *done) 
     return ok();
 }
 
+// Row-major n x dim positions of float4 records to a host buffer. The copy flags
+// a non-finite coordinate on the device (one word back, not a host pass over
+// every coordinate).
+static int export_positions(uint32_t n, int dim, const float4 *pos, cudaStream_t s, float *out) {
+    const size_t count = (size_t)n * dim;
+    float *d = nullptr;
+    CU(cudaMallocAsync((void **)&d, count * 4 + 4, s));
+    uint32_t *flag = (uint32_t *)(d + count);
+    cudaMemsetAsync(flag, 0, 4, s);
+    if (dim == 3)
+        k_export<3><<<div_up(n, 256), 256, 0, s>>>(n, pos, d, flag);
+    else
+        k_export<2><<<div_up(n, 256), 256, 0, s>>>(n, pos, d, flag);
+    uint32_t bad = 0;
+    cudaMemcpyAsync(out, d, count * 4, cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(&bad, flag, 4, cudaMemcpyDeviceToHost, s);
+    cudaFreeAsync(d, s);
+    CU(cudaStreamSynchronize(s));
+    if (bad) return set_err(GR_LAYOUT_FAILED, "non-finite position (StageError::NonFinite)");
+    return ok();
+}
+
 // ------------------------------------------------------------------ ABI -----
 
 extern "C" {
@@ -1121,24 +1143,7 @@ int gr_fa2_positions(gr_fa2 *h, float *out) {
     if (!h) return set_err(GR_INVALID_HANDLE, "null handle");
     if (!out) return set_err(GR_INVALID_ARGUMENT, "out is null");
     if (h->n == 0) return ok();
-    // the copy flags a non-finite coordinate on the device (one word back, not a
-    // host pass over every coordinate)
-    const size_t count = (size_t)h->n * h->dim;
-    float *d = nullptr;
-    CU(cudaMallocAsync((void **)&d, count * 4 + 4, h->stream));
-    uint32_t *flag = (uint32_t *)(d + count);
-    cudaMemsetAsync(flag, 0, 4, h->stream);
-    if (h->dim == 3)
-        k_export<3><<<div_up(h->n, 256), 256, 0, h->stream>>>(h->n, h->pos, d, flag);
-    else
-        k_export<2><<<div_up(h->n, 256), 256, 0, h->stream>>>(h->n, h->pos, d, flag);
-    uint32_t bad = 0;
-    cudaMemcpyAsync(out, d, count * 4, cudaMemcpyDeviceToHost, h->stream);
-    cudaMemcpyAsync(&bad, flag, 4, cudaMemcpyDeviceToHost, h->stream);
-    cudaFreeAsync(d, h->stream);
-    CU(cudaStreamSynchronize(h->stream));
-    if (bad) return set_err(GR_LAYOUT_FAILED, "non-finite position (StageError::NonFinite)");
-    return ok();
+    return export_positions(h->n, h->dim, h->pos, h->stream, out);
 }
 
 int gr_fa2_set_positions(gr_fa2 *h, const float *pos) {
@@ -2707,16 +2712,8 @@ int gr_force_session_tick_timed(gr_force_session *S, uint32_t ticks, float *ms) 
 int gr_force_session_positions(gr_force_session *S, float *out) {
     if (!S) return set_err(GR_INVALID_HANDLE, "null session");
     if (!out && S->n) return set_err(GR_INVALID_ARGUMENT, "out is null");
-    std::vector<float4> host(S->n);
-    if (S->n) CU(cudaMemcpyAsync(host.data(), S->p4, (size_t)S->n * sizeof(float4), cudaMemcpyDeviceToHost, S->t->stream));
-    CU(cudaStreamSynchronize(S->t->stream));
-    for (uint32_t i = 0; i < S->n; i++) {
-        out[2 * (size_t)i] = host[i].x;
-        out[2 * (size_t)i + 1] = host[i].y;
-        if (!std::isfinite(host[i].x) || !std::isfinite(host[i].y))
-            return set_err(GR_LAYOUT_FAILED, "non-finite position (StageError::NonFinite)");
-    }
-    return ok();
+    if (S->n == 0) return ok();
+    return export_positions(S->n, 2, S->p4, S->t->stream, out);
 }
 
 int gr_force_session_velocities(gr_force_session *S, float *out) {
