@@ -226,34 +226,19 @@ k_adj_walk(WalkParams P, const DevState *__restrict__ st, Cells cells, const flo
     const uint32_t lane = threadIdx.x % GR_WARP;
     uint32_t k = 0;
     while (k < ncells) {
-        const float4 A = cell_a<D>(cells, k);
-        const float4 B = cell_b<D>(cells, k);
-        int32_t sk;
-        uint32_t start;
-        float cx, cy, cz, cm, w2, ox, oy, oz;
-        if (D == 2) {
-            cx = A.x; cy = A.y; cz = 0.f; cm = A.z; w2 = A.w;
-            ox = B.x; oy = B.y; oz = 0.f;
-            sk = __float_as_int(B.z);
-            start = __float_as_uint(B.w);
-        } else {
-            const int2 Cc = cell_c3(cells, k);
-            cx = A.x; cy = A.y; cz = A.z; cm = A.w;
-            ox = B.x; oy = B.y; oz = B.z; w2 = B.w;
-            sk = Cc.x;
-            start = (uint32_t)Cc.y;
-        }
-        const bool leaf = sk < 0;
-        uint32_t skip = leaf ? k + 1 : (uint32_t)sk;
-        if (skip <= k || skip > ncells) skip = k + 1;
+        CellRec<D> R = cell_rec<D, false>(cells, k);
+        if (cells.skip) R.skip = cells.skip[k];
+        const uint32_t skip = min(max(R.skip, k + 1), ncells);
+        const bool one = R.w2 < 0.f, leaf = one || R.multi;
+        const float cm = R.m;
         const bool active = resume <= k;
         const bool holds = (k <= mylp) && (mylp < skip);
-        const float dx = (me.x - cx) - ox, dy = (me.y - cy) - oy, dz = (D == 3) ? (me.z - cz) - oz : 0.f;
-        const float d2 = (D == 3) ? dx * dx + dy * dy + dz * dz : dx * dx + dy * dy;
-        const bool far = active && !holds && d2 > 0.f && w2 < th2 * d2;
+        float dx, dy, dz, d2;
+        cell_offset<D>(R, f2_pack(me.x, me.y), me.z, dx, dy, dz, d2);
+        const bool far = active && !holds && d2 > 0.f && fabsf(R.w2) < th2 * d2;
         const bool open = active && !far;
         // a one-point leaf's pair is its body term (the point is its own centre)
-        const bool body = far || (sk == -1 && open && !holds && d2 > 0.f);
+        const bool body = far || (one && open && !holds && d2 > 0.f);
         float jx = 0.f, jy = 0.f, jz = 0.f;
         if (body) {
             rep_jac<D>(kr * me.w * cm, dx, dy, dz, vx, vy, vz, jx, jy, jz);
@@ -276,14 +261,12 @@ k_adj_walk(WalkParams P, const DevState *__restrict__ st, Cells cells, const flo
                 if (D == 3) atomicAdd(&xbar[(size_t)k * D + 2], -(double)jz);
             }
         }
-        if (sk == -1) {
+        if (one) {
             k = k + 1;
         } else if (leaf) {
             if (__any_sync(GR_FULL, open)) {
-                int32_t cnt = -sk;
-                if (start >= n || (uint32_t)cnt > n - start) cnt = 0;
-                for (int32_t q = 0; q < cnt; q++) {
-                    const uint32_t jp = start + (uint32_t)q;
+                const uint2 range = __ldg(&cells.range[k]);
+                for (uint32_t jp = range.x; jp < min(range.y, n); jp++) {
                     const float4 o = __ldg(&sp[jp]);
                     if (open && jp != p) {
                         const float ex = me.x - o.x, ey = me.y - o.y, ez = (D == 3) ? me.z - o.z : 0.f;

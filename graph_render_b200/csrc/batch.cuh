@@ -55,7 +55,7 @@ __host__ __device__ inline T *slot_take(unsigned char *base, size_t &off, size_t
 }
 
 // Lays a slot out for graphs of up to nmax nodes; returns the bytes used.
-__host__ __device__ inline size_t slot_carve(unsigned char *base, uint32_t nmax, int D, SlotView &v) {
+__host__ __device__ inline size_t slot_carve(unsigned char *base, uint32_t nmax, int D, bool wide, SlotView &v) {
     size_t off = 0;
     const size_t n = nmax;
     v.keys = slot_take<uint64_t>(base, off, n);
@@ -87,7 +87,12 @@ __host__ __device__ inline size_t slot_carve(unsigned char *base, uint32_t nmax,
     v.bt.marks = nullptr;
     v.pre = slot_take<BodyDD>(base, off, n + 1);
     v.cell_flag = slot_take<uint8_t>(base, off, n);
-    v.cells = cells_view(slot_take<float4>(base, off, cells_float4s(2 * nmax, D)), 2 * nmax, D);
+    v.cells.a = slot_take<float4>(base, off, 2 * n * (D == 3 ? 2 : 1));
+    v.cells.b = D == 3 ? nullptr : slot_take<float2>(base, off, 2 * n);
+    v.cells.range = slot_take<uint2>(base, off, 2 * n);
+    v.cells.start = nullptr;
+    v.cells.skip = nullptr;
+    if (wide) v.cells.skip = slot_take<uint32_t>(base, off, 2 * n);
     v.rep = slot_take<float>(base, off, n * D);
     v.U = slot_take<float>(base, off, n * D);
     v.att = slot_take<float>(base, off, n * D);
@@ -348,7 +353,8 @@ struct BatchOcc {
     static constexpr int MIN_BLOCKS = BT == 512 ? 3 : BT == 256 ? 4 : 1;
 };
 
-template <int D, int BT>
+// WIDE: the largest graph's tree keeps skip in an array of its own (tree.cuh).
+template <int D, int BT, bool WIDE = false>
 __global__ void __launch_bounds__(BT, BatchOcc<BT>::MIN_BLOCKS) k_batch(BatchArgs A) {
     constexpr int W = BT / GR_WARP;
     __shared__ uint32_t s_cnt[W][256];
@@ -365,7 +371,7 @@ __global__ void __launch_bounds__(BT, BatchOcc<BT>::MIN_BLOCKS) k_batch(BatchArg
 
     const int t = threadIdx.x, lane = t % GR_WARP, w = t / GR_WARP;
     SlotView S;
-    slot_carve(A.slots + (size_t)blockIdx.x * A.slot_bytes, A.nmax, D, S);
+    slot_carve(A.slots + (size_t)blockIdx.x * A.slot_bytes, A.nmax, D, WIDE, S);
 
     for (;;) {
         if (t == 0) {
@@ -507,7 +513,7 @@ __global__ void __launch_bounds__(BT, BatchOcc<BT>::MIN_BLOCKS) k_batch(BatchArg
                     bool coinc;
                     const Body body = leaf_sum<D>(S.sp, a0, a1, coinc);
                     const int level = nu == 1 ? 0 : coinc ? S.bt.delta[S.bt.leaf_parent[s]] / D + 1 : L;
-                    write_cell<D>(S.cells, idx, body, level, s_root_w, -(int32_t)(a1 - a0), a0,
+                    write_cell<D>(S.cells, idx, body, level, s_root_w, idx + 1, a0, a1 - a0,
                                   a1 - a0 == 1 ? &one : nullptr);
                     S.leaf_pre[s] = idx;
                 }
@@ -521,30 +527,29 @@ __global__ void __launch_bounds__(BT, BatchOcc<BT>::MIN_BLOCKS) k_batch(BatchArg
                         atomicOr(&s_st.error, (uint32_t)ERR_TREE);
                         continue;
                     }
-                    write_cell<D>(S.cells, idx, range_body(S.pre[f], S.pre[end]), lv, s_root_w, (int32_t)skip,
-                                  S.leaf_start[f]);
+                    write_cell<D>(S.cells, idx, range_body(S.pre[f], S.pre[end]), lv, s_root_w, skip,
+                                  S.leaf_start[f], 0u);
                 }
             }
             __syncthreads();
             // ---- repulsion walk: warp w takes groups of 32 sorted nodes, one per lane
-            //      (walk_lane: the same forces, bit for bit, as the warp-union walk)
+            //      (walk_own: the one-graph engine's forces, bit for bit)
             {
                 WalkView V{S.cells, S.sp, S.sorig, S.uid, S.leaf_pre, n, ncells, s_st.iter_no, G.seed, G.kr, G.th2,
                            &s_st.error};
                 uint32_t far_acc = 0, pair_acc = 0;
                 for (uint32_t base = (uint32_t)w * GR_WARP; base < n; base += BT) {
-                    float f0, f1, f2;
-                    uint32_t nf, np_;
-                    walk_lane<D>(V, base + lane, f0, f1, f2, nf, np_);
-                    const uint32_t p = base + lane;
-                    if (p < n) {
-                        const uint32_t oi = S.sorig[p];
-                        S.rep[(size_t)oi * D] = f0;
-                        S.rep[(size_t)oi * D + 1] = f1;
-                        if (D == 3) S.rep[(size_t)oi * D + 2] = f2;
+                    WalkNode X;
+                    node_init<D>(V, base + lane, X);
+                    walk_own<D, true, WIDE>(V, X);
+                    if (X.p < n) {
+                        const uint32_t oi = S.sorig[X.p];
+                        S.rep[(size_t)oi * D] = X.f0;
+                        S.rep[(size_t)oi * D + 1] = X.f1;
+                        if (D == 3) S.rep[(size_t)oi * D + 2] = X.f2_;
                     }
-                    far_acc += nf;
-                    pair_acc += np_;
+                    far_acc += X.nfar;
+                    pair_acc += X.npair;
                 }
                 far_acc = __reduce_add_sync(GR_FULL, far_acc);
                 pair_acc = __reduce_add_sync(GR_FULL, pair_acc);

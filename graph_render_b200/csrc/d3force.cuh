@@ -194,8 +194,7 @@ __device__ __forceinline__ bool d3_settle(const D3Params &P, uint32_t tick, uint
 }
 
 // Many-body: per sorted node, the stackless preorder walk of charge.rs
-// node_delta over the cells (A {cx, cy, count, w^2}, B {cx_lo, cy_lo, skip |
-// -count, start}); the delta goes onto the node's own velocity. A cell the
+// node_delta over the cells (their mass is their point count); the delta goes onto the node's own velocity. A cell the
 // opening test resolves acts as one body of its count; a leaf it does not takes
 // its points directly, every point at the leaf centre's offset (charge.rs
 // direct), which is the same term with the count less this node when it lies in
@@ -214,18 +213,20 @@ k_d3_charge(D3Params P, const D3State *st, const DevState *ts, Cells cells, cons
     float ax = 0.f, ay = 0.f;
     uint32_t k = 0;
     while (k < ncells) {
-        const float4 A = cell_a<2>(cells, k);
-        const float4 B = cell_b<2>(cells, k);
-        const int32_t sk = __float_as_int(B.z);
-        const bool leaf = sk < 0;
-        float dx = (A.x - me.x) + B.x, dy = (A.y - me.y) + B.y;
+        CellRec<2> R = cell_rec<2, false>(cells, k);
+        if (cells.skip) R.skip = __ldg(&cells.skip[k]);
+        const bool multi = R.multi, leaf = multi || R.w2 < 0.f;
+        // the displacement to the centre: the records hold it negated
+        float dx = -((me.x + R.a.x) + R.lx), dy = -((me.y + R.a.y) + R.ly);
         float l = dx * dx + dy * dy;
-        const bool open = A.w >= P.th2 * l;  // open >= l: w^2 / theta^2 >= l
-        const bool in_range = l < P.dmax2;   // settle: nothing at or past distanceMax
-        const uint32_t start = __float_as_uint(B.w), cnt = leaf ? (uint32_t)(-sk) : 0u;
-        const bool self_in = leaf && p - start < cnt;  // this node is one of the leaf's points
-        if (dx == 0.f || dy == 0.f) {  // the jiggle, keyed on the chain head (direct) or the cell (body)
-            const uint32_t key = (open && leaf) ? __ldg(&sorig[start + cnt - 1]) : k;
+        const bool open = fabsf(R.w2) >= P.th2 * l;  // open >= l: w^2 / theta^2 >= l
+        const bool in_range = l < P.dmax2;           // settle: nothing at or past distanceMax
+        bool self_in = false;  // this node is one of the leaf's points
+        if (multi || dx == 0.f || dy == 0.f) {  // this node is in no other leaf
+            const uint32_t start = __ldg(&cells.start[k]), last = multi ? __ldg(&cells.range[k].y) - 1u : start;
+            self_in = leaf && p >= start && p <= last;
+            // the jiggle, keyed on the chain head (direct) or the cell (body)
+            const uint32_t key = (open && leaf) ? __ldg(&sorig[last]) : k;
             if (dx == 0.f) {
                 dx = (float)jiggle(P.seed, tick, 2, oi, key);
                 l += dx * dx;
@@ -239,11 +240,11 @@ k_d3_charge(D3Params P, const D3State *st, const DevState *ts, Cells cells, cons
         l = l == 0.f ? fmaxf(P.dmin2, 1.17549435e-38f) : l;
         const bool descend = open && !leaf;
         const bool counted = !descend && in_range;
-        const float m = (open && self_in) ? A.z - 1.f : A.z;
+        const float m = (open && self_in) ? R.m - 1.f : R.m;
         const float f = counted ? m * ca / l : 0.f;
         ax += dx * f;
         ay += dy * f;
-        k = (descend || leaf) ? k + 1 : max((uint32_t)sk, k + 1);
+        k = descend ? k + 1 : max(R.skip, k + 1);
     }
     float2 w = v[oi];
     w.x += ax;

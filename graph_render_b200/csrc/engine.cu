@@ -18,6 +18,7 @@
 #include <cstring>
 #include <mutex>
 #include <new>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/graph_cuda.h"
@@ -125,6 +126,7 @@ struct gr_fa2 {
     double prm[16];
     cudaStream_t stream = nullptr;
     bool own_stream = false;
+    bool session = false;  // holds a d3-force session's tree: its cells keep their starts
 
     // graph
     uint32_t *rp = nullptr, *col = nullptr;
@@ -267,9 +269,12 @@ static cudaError_t alloc_tick_buffers(gr_fa2 *h) {
     A(h->tile_carry, div_up(n, AG_TILE) + 1);
     A(h->tile_cnt, 2 * ((size_t)div_up(n, AG_TILE) + 1));
     {
-        float4 *cb = nullptr;  // cells: 2n at most
-        A(cb, cells_float4s(2 * n, D));
-        h->cells = cells_view(cb, 2 * n, D);
+        const size_t nc = 2 * (size_t)n;  // cells, at most
+        A(h->cells.a, nc * (D == 3 ? 2 : 1));
+        if (D == 2) A(h->cells.b, nc);
+        A(h->cells.range, nc);
+        if (h->session) A(h->cells.start, nc);
+        if (cells_wide(n)) A(h->cells.skip, nc);
     }
     A(h->rep, (size_t)n * D);
     A(h->U, (size_t)n * D);
@@ -488,18 +493,22 @@ template <int D, bool COUNT>
 static void launch_walk(gr_fa2 *h, const WalkParams &wp, cudaStream_t s, bool pdl) {
     const uint32_t n = h->n;
     DevState *st = h->st;
-    if (h->walk_schedule == 3)  // 64 nodes per warp: two groups of 32, one walk of each per lane
-        gr_launch(pdl, k_walk_s<D, 3, COUNT>, div_up(n, 2 * WALK_THREADS), WALK_THREADS, 0, s, wp, st, h->cells,
-                  h->sp, h->sorig, h->uid, h->leaf_pre, h->rep, st);
+    auto launch = [&](auto k, uint32_t nodes) {  // nodes: a lane's
+        gr_launch(pdl, k, div_up(div_up(n, nodes), WALK_THREADS), WALK_THREADS, 0, s, wp, st, h->cells, h->sp, h->sorig,
+                  h->uid, h->leaf_pre, h->rep, st);
+    };
+    if (h->cells.skip && h->walk_schedule == 2)
+        launch(k_walk_s<D, 2, COUNT, true>, 2);
+    else if (h->cells.skip)
+        launch(k_walk_s<D, 1, COUNT, true>, 1);
+    else if (h->walk_schedule == 3)
+        launch(k_walk_s<D, 3, COUNT, false>, 4);
     else if (h->walk_schedule == 2)
-        gr_launch(pdl, k_walk_s<D, 2, COUNT>, div_up(div_up(n, 2), WALK_THREADS), WALK_THREADS, 0, s, wp, st,
-                  h->cells, h->sp, h->sorig, h->uid, h->leaf_pre, h->rep, st);
+        launch(k_walk_s<D, 2, COUNT, false>, 2);
     else if (h->walk_schedule == 1)
-        gr_launch(pdl, k_walk_s<D, 1, COUNT>, div_up(n, WALK_THREADS), WALK_THREADS, 0, s, wp, st, h->cells, h->sp,
-                  h->sorig, h->uid, h->leaf_pre, h->rep, st);
+        launch(k_walk_s<D, 1, COUNT, false>, 1);
     else
-        gr_launch(pdl, k_walk_s<D, 0, COUNT>, div_up(n, WALK_THREADS), WALK_THREADS, 0, s, wp, st, h->cells, h->sp,
-                  h->sorig, h->uid, h->leaf_pre, h->rep, st);
+        launch(k_walk_s<D, 0, COUNT, false>, 1);
 }
 
 template <int D>
@@ -803,7 +812,8 @@ struct SeededStarts {
 
 static int create_impl(gr_fa2 **out, uint32_t n, uint64_t m, const uint32_t *src, const uint32_t *dst,
                        const double *weight, const uint8_t *params, size_t params_len, const float *pos0,
-                       bool tick_buffers = true, SeededStarts starts = SeededStarts()) {
+                       bool tick_buffers = true, SeededStarts starts = SeededStarts(),
+                       bool session = false) {
     if (!out) return set_err(GR_INVALID_ARGUMENT, "out is null");
     *out = nullptr;
     double prm[16];
@@ -820,6 +830,7 @@ static int create_impl(gr_fa2 **out, uint32_t n, uint64_t m, const uint32_t *src
     // the autotuner's choice on both 1M-node graphs: per lane in 2D, two nodes per
     // lane over the union of their walks in 3D (0.43 against 0.46 ms)
     h->walk_schedule = D == 3 ? 2 : 1;
+    h->session = session;
     h->sort_passes = sort_passes_for(n);
     memcpy(h->prm, prm, sizeof prm);
     int rc = GR_OK;
@@ -1523,7 +1534,9 @@ static int forces_static(uint32_t n, const float4 *nodes, const uint32_t *rp, co
     h.tile_sum = cv.take<Body>(div_up(n, AG_TILE) + 1);
     h.tile_carry = cv.take<BodyDD>(div_up(n, AG_TILE) + 1);
     h.tile_cnt = cv.take<uint32_t>(2 * ((size_t)div_up(n, AG_TILE) + 1));
-    h.cells = cells_view(cv.take<float4>(cells_float4s(2 * n, D)), 2 * n, D);
+    h.cells.a = cv.take<float4>(2 * (size_t)n * (D == 3 ? 2 : 1));
+    if (D == 2) h.cells.b = cv.take<float2>(2 * (size_t)n);
+    h.cells.range = cv.take<uint2>(2 * (size_t)n);
     h.rep = cv.take<float>((size_t)n * D);
     h.part = cv.take<double>(std::max<size_t>((size_t)h.bnd_blocks() * 3 * D, 2 * (size_t)div_up(n, FRC_THREADS)) + 8);
     h.sorter.cap = n;
@@ -1638,29 +1651,40 @@ struct gr_fa2_batch {
     }
 };
 
-template <int D, int BT>
+template <int D, int BT, bool WIDE>
 static int batch_slots(uint32_t *slots) {
     int dev = 0, sms = 0, per = 0;
     CU(cudaGetDevice(&dev));
     CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_batch<D, BT>, BT, 0));
+    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_batch<D, BT, WIDE>, BT, 0));
     *slots = (uint32_t)std::max(1, per) * (uint32_t)sms;
     return GR_OK;
 }
 
-static int batch_slots_for(int dim, int bt, uint32_t *slots) {
-    if (dim == 3) {
-        if (bt == 256) return batch_slots<3, 256>(slots);
-        if (bt == 1024) return batch_slots<3, 1024>(slots);
-        return batch_slots<3, 512>(slots);
-    }
-    if (bt == 256) return batch_slots<2, 256>(slots);
-    if (bt == 1024) return batch_slots<2, 1024>(slots);
-    return batch_slots<2, 512>(slots);
+// Calls f with the batch kernel's template arguments: dim, CTA size, and whether
+// the largest graph's tree is wide (then one CTA size, 1,024).
+template <typename F>
+static auto batch_kernel(int dim, int bt, bool wide, F f) {
+    using std::integral_constant;
+    using T = integral_constant<bool, true>;
+    using N = integral_constant<bool, false>;
+    auto with_dim = [&](auto d) {
+        if (wide) return f(d, integral_constant<int, 1024>(), T());
+        if (bt == 256) return f(d, integral_constant<int, 256>(), N());
+        if (bt == 1024) return f(d, integral_constant<int, 1024>(), N());
+        return f(d, integral_constant<int, 512>(), N());
+    };
+    return dim == 3 ? with_dim(integral_constant<int, 3>()) : with_dim(integral_constant<int, 2>());
 }
 
-template <int D, int BT>
-static void batch_launch(gr_fa2_batch *b, uint32_t ticks, uint32_t slots) {
+static int batch_slots_for(int dim, int bt, bool wide, uint32_t *slots) {
+    return batch_kernel(dim, bt, wide, [&](auto d, auto t, auto w) {
+        return batch_slots<decltype(d)::value, decltype(t)::value, decltype(w)::value>(slots);
+    });
+}
+
+template <int D, int BT, bool WIDE>
+static int batch_launch(gr_fa2_batch *b, uint32_t ticks, uint32_t slots) {
     BatchArgs a;
     a.graphs = b->d_graphs;
     a.state = b->d_state;
@@ -1677,23 +1701,18 @@ static void batch_launch(gr_fa2_batch *b, uint32_t ticks, uint32_t slots) {
     a.nmax = b->nmax;
     a.ticks = ticks;
     cudaMemsetAsync(b->d_next, 0, sizeof(uint32_t), b->g->stream);
-    k_batch<D, BT><<<slots, BT, 0, b->g->stream>>>(a);
+    k_batch<D, BT, WIDE><<<slots, BT, 0, b->g->stream>>>(a);
+    return GR_OK;
 }
 
 static int batch_enqueue(gr_fa2_batch *b, uint32_t ticks) {
     uint32_t slots = 0;
-    if (int c = batch_slots_for(b->dim, b->threads, &slots)) return c;
+    const bool wide = cells_wide(b->nmax);
+    if (int c = batch_slots_for(b->dim, b->threads, wide, &slots)) return c;
     slots = std::min(slots, b->max_slots);
-    if (b->dim == 3) {
-        if (b->threads == 256) batch_launch<3, 256>(b, ticks, slots);
-        else if (b->threads == 1024) batch_launch<3, 1024>(b, ticks, slots);
-        else batch_launch<3, 512>(b, ticks, slots);
-    } else {
-        if (b->threads == 256) batch_launch<2, 256>(b, ticks, slots);
-        else if (b->threads == 1024) batch_launch<2, 1024>(b, ticks, slots);
-        else batch_launch<2, 512>(b, ticks, slots);
-    }
-    return GR_OK;
+    return batch_kernel(b->dim, b->threads, wide, [&](auto d, auto t, auto w) {
+        return batch_launch<decltype(d)::value, decltype(t)::value, decltype(w)::value>(b, ticks, slots);
+    });
 }
 
 static int batch_run_impl(gr_fa2_batch *b, uint32_t ticks, float *ms) {
@@ -1849,7 +1868,7 @@ int gr_fa2_batch_create(gr_fa2_batch **out, uint32_t ngraphs, const uint32_t *no
     uint32_t slots = 0;
     for (int bt : {256, 512, 1024}) {
         uint32_t sl = 0;
-        if (int c = batch_slots_for(dim, bt, &sl)) {
+        if (int c = batch_slots_for(dim, bt, cells_wide(nmax), &sl)) {
             delete b;
             return c;
         }
@@ -1857,7 +1876,7 @@ int gr_fa2_batch_create(gr_fa2_batch **out, uint32_t ngraphs, const uint32_t *no
     }
     slots = std::min(slots, ngraphs);
     SlotView sv;
-    b->slot_bytes = slot_carve(nullptr, nmax, dim, sv);
+    b->slot_bytes = slot_carve(nullptr, nmax, dim, cells_wide(nmax), sv);
     b->max_slots = slots;
     cudaError_t ce;
     if ((ce = cudaMalloc(&b->d_graphs, ngraphs * sizeof(BatchGraph))) ||
@@ -2600,7 +2619,7 @@ int gr_force_session_create(gr_force_session **out, uint32_t n, uint64_t m, cons
     uint8_t fb[sizeof fv];
     memcpy(fb, fv, sizeof fv);
     gr_fa2 *t = nullptr;
-    if (int c = create_impl(&t, n, m, src, dst, strength, fb, sizeof fb, nullptr)) return c;
+    if (int c = create_impl(&t, n, m, src, dst, strength, fb, sizeof fb, nullptr, true, SeededStarts(), true)) return c;
     gr_force_session *S = new (std::nothrow) gr_force_session();
     if (!S) {
         delete t;

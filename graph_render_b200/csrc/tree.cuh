@@ -970,48 +970,74 @@ __device__ __forceinline__ bool is_cell(const BinTree &t, int32_t node) {
     return par < 0 || (t.delta[node] / D) != (t.delta[par] / D);
 }
 
-// Cell record, 2D: A = {cx, cy, mass, w^2}, B = {cx_lo, cy_lo, skip | -count, start}.
-// 3D: A = {cx, cy, cz, mass}, B = {cx_lo, cy_lo, cz_lo, w^2}, C = {skip | -count, start, -, -}.
+// Cell record, 2D: a = {-cx, -cy, -cx_lo, -cy_lo}, b = {mass, word}.
+// 3D: a[2k] = {-cx, -cy, -cz, mass}, a[2k + 1] = {-cx_lo, -cy_lo, -cz_lo, word}.
 // The centre is an FP32 hi/lo pair of the FP64 centre of mass, so a node at
-// 1e4 still resolves a nearby centre to ~1e-3 ulp instead of a whole FP32 ulp.
-// In 2D the A and B records are two arrays (rec[k], rec_b[k]): the 32 lanes of a
-// walk warp visit different but nearby cells, and one 32-byte sector of the A
-// array holds two cells' A (measured: a per-cell 32-byte record made the 2D
-// per-lane walk 13% slower). In 3D a cell's records lie together (rec[3k + 0] =
-// A, + 1 = B, + 2 = C): one line per visit instead of three (the 3D walk 6%
-// faster than with three arrays).
-template <int D> struct CellF { static constexpr uint32_t F = D == 3 ? 3 : 1; };  // float4s per cell in rec
+// 1e4 still resolves a nearby centre to ~1e-3 ulp instead of a whole FP32 ulp;
+// it is stored negated, so that a displacement is two packed additions.
+// A walk is bound by the bytes its lanes gather through the L1 (ncu, 1M nodes in
+// 2D with records of 32 bytes: 86% of the data pipe's wavefronts, 6.6 a request),
+// so the rest of a record is one word: w^2 is a power of two (the root's side is),
+// and its exponent stands where a float's does, under a sign bit that is set in a
+// leaf of one point, which acts as a body at any distance; the low 23 bits are
+// skip, the cell to go on with once this one is done (k + 1 for a leaf). A
+// negative mass marks a leaf of several points, whose range of them is beside. Trees of more than CELL_SKIP cells keep skip in an array of its own.
+// In 2D the a and b records are two arrays: the 32 lanes of a walk warp visit
+// different but nearby cells, and a 32-byte sector holds several cells' records
+// (measured: a per-cell record of both made the 2D per-lane walk 13% slower).
+constexpr uint32_t CELL_SKIP = 0x3fffffu, CELL_MULTI = 0x400000u, CELL_W2 = 0xff800000u;
 
 struct Cells {
-    float4 *rec;     // 2D: A of cell k at rec[k]; 3D: cell k's A, B, C at rec[3k ..]
-    float4 *rec_b;   // 2D: B of cell k at rec_b[k]; 3D: unused
+    float4 *a;
+    float2 *b;        // 2D only
+    uint2 *range;     // a leaf of several points: its first and one-past-last sorted point (others unwritten)
+    uint32_t *start;  // nullable: every cell's first sorted point
+    uint32_t *skip;   // null: in the records
 };
 
+// Whether a graph of n nodes (2n cells at most) keeps skip in an array of its own.
+__host__ __device__ inline bool cells_wide(uint32_t n) { return n > CELL_SKIP / 2; }
+
+// One cell's records as a walk reads them. WIDE: skip has its own array.
 template <int D>
-__device__ __forceinline__ float4 cell_a(const Cells &c, uint32_t k) {
-    return __ldg(&c.rec[(size_t)k * CellF<D>::F]);
-}
-template <int D>
-__device__ __forceinline__ float4 cell_b(const Cells &c, uint32_t k) {
-    return D == 3 ? __ldg(&c.rec[(size_t)k * 3 + 1]) : __ldg(&c.rec_b[k]);
-}
-__device__ __forceinline__ int2 cell_c3(const Cells &c, uint32_t k) {  // 3D: {skip | -count, start}
-    const float4 v = __ldg(&c.rec[(size_t)k * 3 + 2]);
-    return make_int2(__float_as_int(v.x), __float_as_int(v.y));
+struct CellRec {
+    float4 a;
+    float lx, ly, lz, m, w2;
+    uint32_t skip;
+    bool multi;
+};
+
+template <int D, bool WIDE>
+__device__ __forceinline__ CellRec<D> cell_rec(const Cells &c, uint32_t k) {
+    CellRec<D> r;
+    uint32_t word;
+    if (D == 2) {
+        r.a = __ldg(&c.a[k]);
+        const float2 B = __ldg(&c.b[k]);
+        r.lx = r.a.z;
+        r.ly = r.a.w;
+        r.lz = 0.f;
+        r.m = B.x;
+        word = __float_as_uint(B.y);
+    } else {
+        r.a = __ldg(&c.a[2 * (size_t)k]);
+        const float4 B = __ldg(&c.a[2 * (size_t)k + 1]);
+        r.lx = B.x;
+        r.ly = B.y;
+        r.lz = B.z;
+        r.m = r.a.w;
+        word = __float_as_uint(B.w);
+    }
+    r.w2 = __uint_as_float(word & CELL_W2);
+    r.multi = (word & CELL_MULTI) != 0u;
+    r.skip = WIDE ? __ldg(&c.skip[k]) : word & CELL_SKIP;
+    return r;
 }
 
-// Float4 records a cells buffer holds for `cap` cells, and its two views.
-__host__ __device__ inline size_t cells_float4s(uint32_t cap, int dim) { return (size_t)cap * (dim == 3 ? 3 : 2); }
-__host__ __device__ inline Cells cells_view(float4 *buf, uint32_t cap, int dim) {
-    Cells c;
-    c.rec = buf;
-    c.rec_b = dim == 3 ? nullptr : buf + cap;
-    return c;
-}
-
+// leaf: 0 for an internal cell, else its point count.
 template <int D>
 __device__ __forceinline__ void write_cell(Cells c, uint32_t idx, const Body &b, int level, double root_w,
-                                           int32_t skip_or_count, uint32_t start, const float4 *point = nullptr) {
+                                           uint32_t skip, uint32_t start, uint32_t leaf, const float4 *point = nullptr) {
     double inv = 1.0 / b.m;
     double cc[3] = {b.c0 * inv, b.c1 * inv, b.c2 * inv};
     if (point) {  // a one-point leaf's centre is the point itself, exactly
@@ -1025,17 +1051,20 @@ __device__ __forceinline__ void write_cell(Cells c, uint32_t idx, const Body &b,
         hi[a] = (float)cc[a];
         lo[a] = (float)(cc[a] - (double)hi[a]);
     }
-    double w = ldexp(root_w, -level);
-    float w2 = (float)(w * w);
-    float4 *r = c.rec + (size_t)idx * CellF<D>::F;
+    const double w = ldexp(root_w, -level);
+    const uint32_t word = (__float_as_uint((float)(w * w)) & 0x7f800000u) | (leaf == 1 ? 0x80000000u : 0u) |
+                          (leaf > 1 ? CELL_MULTI : 0u) | (c.skip ? 0u : skip & CELL_SKIP);
+    const float m = (float)b.m;
     if (D == 2) {
-        r[0] = make_float4(hi[0], hi[1], (float)b.m, w2);
-        c.rec_b[idx] = make_float4(lo[0], lo[1], __int_as_float(skip_or_count), __uint_as_float(start));
+        c.a[idx] = make_float4(-hi[0], -hi[1], -lo[0], -lo[1]);
+        c.b[idx] = make_float2(m, __uint_as_float(word));
     } else {
-        r[0] = make_float4(hi[0], hi[1], hi[2], (float)b.m);
-        r[1] = make_float4(lo[0], lo[1], lo[2], w2);
-        r[2] = make_float4(__int_as_float(skip_or_count), __uint_as_float(start), 0.f, 0.f);
+        c.a[2 * (size_t)idx] = make_float4(-hi[0], -hi[1], -hi[2], m);
+        c.a[2 * (size_t)idx + 1] = make_float4(-lo[0], -lo[1], -lo[2], __uint_as_float(word));
     }
+    if (leaf > 1) c.range[idx] = make_uint2(start, start + leaf);
+    if (c.start) c.start[idx] = start;
+    if (c.skip) c.skip[idx] = skip;
 }
 
 // Every cell at its preorder index, without walking chains: threads
@@ -1074,7 +1103,7 @@ __global__ void k_assign_cells(const DevState *st, BinTree t, uint32_t n_slots, 
         const Body body = leaf_sum<D>(sp, a0, a1, coinc);
         // the parent's record only for coincident points (one leaf alone is the root)
         const int level = nu == 1 ? 0 : coinc ? t.rec[t.leaf_parent[s]].w / D + 1 : L;
-        write_cell<D>(cells, idx, body, level, rw, -(int32_t)(a1 - a0), a0, a1 - a0 == 1 ? &one : nullptr);
+        write_cell<D>(cells, idx, body, level, rw, idx + 1, a0, a1 - a0, a1 - a0 == 1 ? &one : nullptr);
         leaf_pre[s] = idx;
         return;
     }
@@ -1091,7 +1120,7 @@ __global__ void k_assign_cells(const DevState *st, BinTree t, uint32_t n_slots, 
     }
     const uint32_t a0 = leaf_start[f];
     pre.nu = nu;
-    write_cell<D>(cells, idx, range_body(prefix_at<D>(pre, f), prefix_at<D>(pre, end)), lv, rw, (int32_t)skip, a0);
+    write_cell<D>(cells, idx, range_body(prefix_at<D>(pre, f), prefix_at<D>(pre, end)), lv, rw, skip, a0, 0u);
     if (t.cell_of) t.cell_of[i] = idx;
 }
 

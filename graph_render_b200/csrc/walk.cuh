@@ -6,14 +6,21 @@
 // of its mass and the walk skips its subtree; a leaf that is not far acts pair by
 // pair (with the coincident-pair jiggle, state.rs:185-203); anything else opens.
 //
-// On the GPU a warp walks 32 consecutive Morton-sorted nodes together. The cell
-// index k is warp-uniform; each lane keeps `resume`, the first cell index it
-// takes part in again after it approximated a subtree (its skip). The warp
-// descends (k + 1) when any participating lane opens the cell and jumps to
-// skip otherwise; lanes never see a cell their own walk would not visit, so each
-// node's interaction set is exactly the per-node walk's. Cell loads are
-// warp-uniform broadcasts of float4 records; leaf points come from the sorted
-// float4 node array.
+// On the GPU every node walks the preorder cells without a stack: a far cell's
+// skip, or the next cell. The schedules differ in how lanes share the loads of
+// cells; every node meets its own cells in the same order with the same
+// arithmetic in all of them.
+//
+// What bounds it: the L1's data pipe. A step gathers two records a lane; at 1M
+// nodes in 2D that is 6.6M load instructions of 5.2 wavefronts each, 81% of the
+// pipe's rate (ncu; issue 62%, DRAM a few percent). Records of 24 bytes (tree.cuh)
+// instead of 32, the packed displacement, one reciprocal without a subnormal
+// path and one select for the next cell took the walk alone from 195 us (86% of
+// the pipe, 144M warp instructions) to 163 us (104M); in 3D, two nodes a lane
+// without a branch between them took it from 430 to 325 us beside the attraction.
+// Groups of the four sibling cells tested together (128 bytes a group, a stack
+// per lane) took 372 us: the lanes' walks drift apart and every load spreads over
+// six lines.
 #pragma once
 
 #include "common.cuh"
@@ -21,7 +28,7 @@
 
 namespace gr {
 
-constexpr int WALK_THREADS = 256;  // measured at 1M 2D nodes: 64 and 128 threads slower (by 3.5% / 1.6% of the walk)
+constexpr int WALK_THREADS = 256;  // against 128 and 512 threads 1.5% and 4% less at 1M 2D nodes
 
 struct WalkParams {
     uint32_t n;
@@ -40,427 +47,227 @@ struct WalkView {
     uint32_t *err;
 };
 
-// The whole warp calls this for the sorted nodes p = base + lane (lanes with
-// p >= n take part in the votes only). Returns each lane's repulsion and its
-// far / pair interaction counts.
-template <int D, bool COUNT = true>
-__device__ __forceinline__ void walk_group(const WalkView &V, uint32_t p, float &f0, float &f1, float &f2,
-                                           uint32_t &nfar, uint32_t &npair) {
-    const Cells cells = V.cells;
-    const float4 *__restrict__ sp = V.sp;
-    const uint32_t n = V.n, ncells = V.ncells, iter = V.iter;
-    const bool valid = p < n;
-    const float4 me = valid ? sp[p] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const uint32_t mylp = valid ? V.leaf_pre[V.uid[p]] : 0xffffffffu;
-    const uint32_t oi = valid ? V.sorig[p] : 0u;
-    uint32_t resume = valid ? 0u : 0xffffffffu;
-    f0 = f1 = f2 = 0.f;
-    nfar = npair = 0;
-    const float th2 = V.th2, mk = me.w * V.kr;
-    const uint32_t lane = threadIdx.x % GR_WARP;
+// ---- two FP32 values in one 64-bit register (sm_100 packed arithmetic; each half
+// is rounded as the scalar instruction rounds it)
 
-    uint32_t k = 0;
-    while (k < ncells) {
-        const float4 A = cell_a<D>(cells, k);
-        const float4 B = cell_b<D>(cells, k);
-        int32_t sk;
-        uint32_t start;
-        float cx, cy, cz, cm, w2, lx, ly, lz;
-        if (D == 2) {
-            cx = A.x; cy = A.y; cz = 0.f; cm = A.z; w2 = A.w;
-            lx = B.x; ly = B.y; lz = 0.f;
-            sk = __float_as_int(B.z);
-            start = __float_as_uint(B.w);
-        } else {
-            const int2 Cc = cell_c3(cells, k);
-            cx = A.x; cy = A.y; cz = A.z; cm = A.w;
-            lx = B.x; ly = B.y; lz = B.z; w2 = B.w;
-            sk = Cc.x;
-            start = (uint32_t)Cc.y;
-        }
-        const bool leaf = sk < 0;
-        uint32_t skip = leaf ? k + 1 : (uint32_t)sk;
-        if (skip <= k || skip > ncells) {  // malformed cell: record it, keep the walk finite
-            if (lane == 0) atomicOr(V.err, (uint32_t)ERR_TREE);
-            skip = k + 1;
-        }
-        const bool active = resume <= k;
-        const bool holds = (k <= mylp) && (mylp < skip);
-        const float dx = (me.x - cx) - lx;
-        const float dy = (me.y - cy) - ly;
-        const float dz = (D == 3) ? (me.z - cz) - lz : 0.f;
-        const float d2 = (D == 3) ? dx * dx + dy * dy + dz * dz : dx * dx + dy * dy;
-        const bool far = active && !holds && d2 > 0.f && w2 < th2 * d2;
-        if (far) {
-            const float f = __fdividef(mk * cm, d2);
-            f0 += dx * f;
-            f1 += dy * f;
-            if (D == 3) f2 += dz * f;
-            resume = skip;
-            if (COUNT) nfar++;
-        }
-        const bool open = active && !far;
-        if (sk == -1) {
-            // One-point leaf: the exact pair (barnes_hut.rs:163-184) is the body
-            // term above with the point as its own centre; only an exact
-            // coincidence (d2 == 0) takes repel_delta's jiggle.
-            if (open && !holds) {
-                float ex = dx, ey = dy, ez = dz, e2 = d2;
-                if (!(d2 > 0.f)) {
-                    const uint32_t oj = __ldg(&V.sorig[start]);
-                    const float sg = oi < oj ? 1.f : -1.f;
-                    ex = sg * (float)jiggle(V.seed, iter, 0, oi, oj);
-                    ey = sg * (float)jiggle(V.seed, iter, 1, oi, oj);
-                    if (D == 3) ez = sg * (float)jiggle(V.seed, iter, 2, oi, oj);
-                    e2 = (D == 3) ? ex * ex + ey * ey + ez * ez : ex * ex + ey * ey;
-                }
-                const float f = __fdividef(mk * cm, e2);
-                f0 += ex * f;
-                f1 += ey * f;
-                if (D == 3) f2 += ez * f;
-                if (COUNT) npair++;
-            }
-            k = k + 1;
-        } else if (leaf) {
-            if (__any_sync(GR_FULL, open)) {
-                int32_t cnt = -sk;
-                if (start >= n || (uint32_t)cnt > n - start) {
-                    if (lane == 0) atomicOr(V.err, (uint32_t)ERR_TREE);
-                    cnt = 0;
-                }
-                for (int32_t q = 0; q < cnt; q++) {
-                    const uint32_t jp = start + (uint32_t)q;
-                    const float4 o = __ldg(&sp[jp]);
-                    if (open && jp != p) {
-                        float ex = me.x - o.x, ey = me.y - o.y, ez = (D == 3) ? me.z - o.z : 0.f;
-                        if (ex == 0.f && ey == 0.f && (D == 2 || ez == 0.f)) {
-                            // repel_delta's jiggle, taken from the lower index
-                            const uint32_t oj = __ldg(&V.sorig[jp]);
-                            const float sg = oi < oj ? 1.f : -1.f;
-                            ex = sg * (float)jiggle(V.seed, iter, 0, oi, oj);
-                            ey = sg * (float)jiggle(V.seed, iter, 1, oi, oj);
-                            if (D == 3) ez = sg * (float)jiggle(V.seed, iter, 2, oi, oj);
-                        }
-                        const float e2 = (D == 3) ? ex * ex + ey * ey + ez * ez : ex * ex + ey * ey;
-                        const float f = __fdividef(mk * o.w, e2);
-                        f0 += ex * f;
-                        f1 += ey * f;
-                        if (D == 3) f2 += ez * f;
-                        if (COUNT) npair++;
-                    }
-                }
-            }
-            k = k + 1;
-        } else {
-            k = __any_sync(GR_FULL, open) ? k + 1 : skip;
-        }
-    }
+typedef unsigned long long f2;
+
+__device__ __forceinline__ f2 f2_pack(float a, float b) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
 }
-
-// The same per-node walk with every lane on its own cell index (gathered cell
-// loads, no warp vote): the warp runs as long as its longest path instead of
-// the union of its 32 paths. Each lane meets its cells in the same preorder and
-// adds the same terms in the same order as walk_group, so the forces are
-// bit-identical; only the schedule differs.
-// One node's per-lane walk, as state and one cell visit at a time.
-struct LaneNode {
-    float4 me;
-    uint32_t p, mylp, oi, k;
-    float mk, f0, f1, f2;
-    uint32_t nfar, npair;
-};
-
-template <int D>
-__device__ __forceinline__ void lane_init(const WalkView &V, uint32_t p, LaneNode &X) {
-    const bool valid = p < V.n;
-    X.p = p;
-    X.me = valid ? V.sp[p] : make_float4(0.f, 0.f, 0.f, 0.f);
-    X.mylp = valid ? V.leaf_pre[V.uid[p]] : 0u;
-    X.oi = valid ? V.sorig[p] : 0u;
-    X.mk = X.me.w * V.kr;
-    X.f0 = X.f1 = X.f2 = 0.f;
-    X.nfar = X.npair = 0;
-    X.k = valid ? 0u : V.ncells;
+__device__ __forceinline__ void f2_unpack(f2 v, float &a, float &b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
 }
-
-// One cell's records as the walk reads them (C only in 3D).
-struct CellRec {
-    float4 A, B;
-    int2 C;
-};
-
-template <int D>
-__device__ __forceinline__ CellRec cell_rec(const Cells &cells, uint32_t k) {
-    CellRec r;
-    r.A = cell_a<D>(cells, k);
-    r.B = cell_b<D>(cells, k);
-    r.C = D == 3 ? cell_c3(cells, k) : make_int2(0, 0);
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// 1 / x to an ulp; a subnormal x counts as 0
+__device__ __forceinline__ float rcp_ftz(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
 
-// The visit of cell X.k (X.k < ncells) whose records are R: a body term, a
-// leaf's pairs, or a descent; X.k moves on. COUNT: keep the far / pair
-// interaction counts.
-template <int D, bool COUNT = true>
-__device__ __forceinline__ void lane_visit(const WalkView &V, LaneNode &X, const CellRec &R) {
-    const float4 *__restrict__ sp = V.sp;
-    const uint32_t n = V.n, iter = V.iter, k = X.k, oi = X.oi;
-    const float4 me = X.me;
-    const float th2 = V.th2, mk = X.mk;
-    const float4 A = R.A;
-    const float4 B = R.B;
-    int32_t sk;
-    uint32_t start;
-    float cx, cy, cz, cm, w2, lx, ly, lz;
-    if (D == 2) {
-        cx = A.x; cy = A.y; cz = 0.f; cm = A.z; w2 = A.w;
-        lx = B.x; ly = B.y; lz = 0.f;
-        sk = __float_as_int(B.z);
-        start = __float_as_uint(B.w);
-    } else {
-        const int2 Cc = R.C;
-        cx = A.x; cy = A.y; cz = A.z; cm = A.w;
-        lx = B.x; ly = B.y; lz = B.z; w2 = B.w;
-        sk = Cc.x;
-        start = (uint32_t)Cc.y;
-    }
-    const bool leaf = sk < 0;
-    // a leaf (sk < 0) moves on to k + 1, a cell to its skip; every step moves
-    // forward, whatever a cell holds (k < ncells <= 2^31)
-    const uint32_t skip = (uint32_t)max(sk, (int32_t)k + 1);
-    const bool holds = (k <= X.mylp) && (X.mylp < skip);
-    const float dx = (me.x - cx) - lx;
-    const float dy = (me.y - cy) - ly;
-    const float dz = (D == 3) ? (me.z - cz) - lz : 0.f;
-    const float d2 = (D == 3) ? dx * dx + dy * dy + dz * dz : dx * dx + dy * dy;
-    const bool far = !holds && w2 < th2 * d2;  // w2 > 0, so this is false at d2 == 0
-    // The common outcomes without a branch: a body term (far cell, or a
-    // one-point leaf's pair) is added, anything else adds +-0 (an exact no-op:
-    // the sums start at +0 and never hold -0); the walk moves to skip or k + 1.
-    const bool body = far || (sk == -1 && !holds && d2 > 0.f);
-    const float fb = __fdividef(mk * cm, d2);
-    const float f = body ? fb : 0.f;
-    X.f0 += dx * f;
-    X.f1 += dy * f;
-    if (D == 3) X.f2 += dz * f;
-    if (COUNT) {
-        X.nfar += far ? 1u : 0u;
-        X.npair += (body && !far) ? 1u : 0u;
-    }
-    if (!leaf || body) {
-        X.k = body ? skip : k + 1;
-    } else if (!holds && sk == -1) {  // coincident one-point leaf: the jiggle
-        const uint32_t oj = __ldg(&V.sorig[start]);
-        const float sg = oi < oj ? 1.f : -1.f;
-        const float ex = sg * (float)jiggle(V.seed, iter, 0, oi, oj);
-        const float ey = sg * (float)jiggle(V.seed, iter, 1, oi, oj);
-        const float ez = (D == 3) ? sg * (float)jiggle(V.seed, iter, 2, oi, oj) : 0.f;
-        const float e2 = (D == 3) ? ex * ex + ey * ey + ez * ez : ex * ex + ey * ey;
-        const float g = __fdividef(mk * cm, e2);
-        X.f0 += ex * g;
-        X.f1 += ey * g;
-        if (D == 3) X.f2 += ez * g;
-        if (COUNT) X.npair++;
-        X.k = k + 1;
-    } else {  // several points (or this node's own leaf): exact pairs
-        int32_t cnt = -sk;
-        if (start >= n || (uint32_t)cnt > n - start) {
-            atomicOr(V.err, (uint32_t)ERR_TREE);
-            cnt = 0;
-        }
-        for (int32_t q = 0; q < cnt; q++) {
-            const uint32_t jp = start + (uint32_t)q;
-            if (jp == X.p) continue;
-            const float4 o = __ldg(&sp[jp]);
-            float ex = me.x - o.x, ey = me.y - o.y, ez = (D == 3) ? me.z - o.z : 0.f;
-            if (ex == 0.f && ey == 0.f && (D == 2 || ez == 0.f)) {
-                const uint32_t oj = __ldg(&V.sorig[jp]);
-                const float sg = oi < oj ? 1.f : -1.f;
-                ex = sg * (float)jiggle(V.seed, iter, 0, oi, oj);
-                ey = sg * (float)jiggle(V.seed, iter, 1, oi, oj);
-                if (D == 3) ez = sg * (float)jiggle(V.seed, iter, 2, oi, oj);
-            }
-            const float e2 = (D == 3) ? ex * ex + ey * ey + ez * ez : ex * ex + ey * ey;
-            const float g = __fdividef(mk * o.w, e2);
-            X.f0 += ex * g;
-            X.f1 += ey * g;
-            if (D == 3) X.f2 += ez * g;
-            if (COUNT) X.npair++;
-        }
-        X.k = k + 1;
+// A node's displacement from the cell's centre and its square.
+template <int D>
+__device__ __forceinline__ void cell_offset(const CellRec<D> &R, f2 xy, float z, float &dx, float &dy, float &dz,
+                                            float &d2) {
+    f2_unpack(f2_add(f2_add(xy, f2_pack(R.a.x, R.a.y)), f2_pack(R.lx, R.ly)), dx, dy);
+    d2 = __fmaf_rn(dx, dx, __fmul_rn(dy, dy));
+    dz = 0.f;
+    if (D == 3) {
+        dz = (z + R.a.z) + R.lz;
+        d2 = __fmaf_rn(dz, dz, d2);
     }
 }
 
-// The visit of cell X.k (X.k < ncells), its records loaded here.
-template <int D, bool COUNT = true>
-__device__ __forceinline__ void lane_step(const WalkView &V, LaneNode &X) {
-    lane_visit<D, COUNT>(V, X, cell_rec<D>(V.cells, X.k));
-}
-
-template <int D, bool COUNT = true>
-__device__ __forceinline__ void walk_lane(const WalkView &V, uint32_t p, float &f0, float &f1, float &f2,
-                                          uint32_t &nfar, uint32_t &npair) {
-    LaneNode X;
-    lane_init<D>(V, p, X);
-    while (X.k < V.ncells) lane_step<D, COUNT>(V, X);
-    f0 = X.f0;
-    f1 = X.f1;
-    f2 = X.f2;
-    nfar = X.nfar;
-    npair = X.npair;
-}
-
-// One node of a two-node walk (walk_pair): its own state and its visit of
-// cell k when k >= resume, with walk_lane's arithmetic.
-struct PairNode {
-    float4 me;
-    uint32_t p, mylp, oi, resume;
-    float mk, f0, f1, f2;
+// One node in its walk: its own coordinates, the preorder index of its leaf, and
+// the sums so far. k: the cell it goes on with (in the union schedules, the first
+// cell it takes part in again).
+struct WalkNode {
+    f2 xy;
+    float z, mk, f0, f1, f2_;
+    uint32_t p, mylp, k;
     uint32_t nfar, npair;
 };
 
 template <int D>
-__device__ __forceinline__ void pair_init(const WalkView &V, uint32_t p, PairNode &X) {
+__device__ __forceinline__ void node_init(const WalkView &V, uint32_t p, WalkNode &X) {
     const bool valid = p < V.n;
+    const float4 me = valid ? V.sp[p] : make_float4(0.f, 0.f, 0.f, 0.f);
     X.p = p;
-    X.me = valid ? V.sp[p] : make_float4(0.f, 0.f, 0.f, 0.f);
+    X.xy = f2_pack(me.x, me.y);
+    X.z = me.z;
+    X.mk = me.w * V.kr;
     X.mylp = valid ? V.leaf_pre[V.uid[p]] : 0u;
-    X.oi = valid ? V.sorig[p] : 0u;
-    X.resume = valid ? 0u : 0xffffffffu;
-    X.mk = X.me.w * V.kr;
-    X.f0 = X.f1 = X.f2 = 0.f;
+    X.f0 = X.f1 = X.f2_ = 0.f;
     X.nfar = X.npair = 0;
+    X.k = valid ? 0u : 0xffffffffu;
 }
 
-template <int D, bool COUNT = true>
-__device__ __forceinline__ void pair_visit(const WalkView &V, PairNode &X, uint32_t k, float cx, float cy, float cz,
-                                           float lx, float ly, float lz, float cm, float w2, int32_t sk,
-                                           uint32_t start, uint32_t skip, bool leaf) {
-    if (k < X.resume) return;  // inside a subtree this node approximated
-    const bool holds = (k <= X.mylp) && (X.mylp < skip);
-    const float dx = (X.me.x - cx) - lx;
-    const float dy = (X.me.y - cy) - ly;
-    const float dz = (D == 3) ? (X.me.z - cz) - lz : 0.f;
-    const float d2 = (D == 3) ? dx * dx + dy * dy + dz * dz : dx * dx + dy * dy;
-    const bool far = !holds && w2 < V.th2 * d2;
-    const bool body = far || (sk == -1 && !holds && d2 > 0.f);
-    const float fb = __fdividef(X.mk * cm, d2);
-    const float f = body ? fb : 0.f;
-    X.f0 += dx * f;
-    X.f1 += dy * f;
-    if (D == 3) X.f2 += dz * f;
-    if (COUNT) {
-        X.nfar += far ? 1u : 0u;
-        X.npair += (body && !far) ? 1u : 0u;
-    }
-    X.resume = body ? skip : k + 1;
-    if (!leaf || body) return;
-    const float4 *__restrict__ sp = V.sp;
-    const uint32_t n = V.n, iter = V.iter;
-    if (!holds && sk == -1) {  // coincident one-point leaf: the jiggle
-        const uint32_t oj = __ldg(&V.sorig[start]);
-        const float sg = X.oi < oj ? 1.f : -1.f;
-        const float ex = sg * (float)jiggle(V.seed, iter, 0, X.oi, oj);
-        const float ey = sg * (float)jiggle(V.seed, iter, 1, X.oi, oj);
-        const float ez = (D == 3) ? sg * (float)jiggle(V.seed, iter, 2, X.oi, oj) : 0.f;
-        const float e2 = (D == 3) ? ex * ex + ey * ey + ez * ez : ex * ex + ey * ey;
-        const float g = __fdividef(X.mk * cm, e2);
-        X.f0 += ex * g;
-        X.f1 += ey * g;
-        if (D == 3) X.f2 += ez * g;
-        if (COUNT) X.npair++;
+// The points of a leaf that is not far, one by one, repel_delta's jiggle for an
+// exact coincidence (state.rs:185-203).
+template <int D>
+__device__ __forceinline__ void node_pairs(const WalkView &V, WalkNode &X, uint2 range) {
+    const uint32_t start = range.x, stop = range.y;
+    if (start >= V.n || stop > V.n || stop <= start) {
+        atomicOr(V.err, (uint32_t)ERR_TREE);
         return;
     }
-    int32_t cnt = -sk;  // several points (or this node's own leaf): exact pairs
-    if (start >= n || (uint32_t)cnt > n - start) {
-        atomicOr(V.err, (uint32_t)ERR_TREE);
-        cnt = 0;
-    }
-    for (int32_t q = 0; q < cnt; q++) {
-        const uint32_t jp = start + (uint32_t)q;
+    float mx, my;
+    f2_unpack(X.xy, mx, my);
+    for (uint32_t jp = start; jp < stop; jp++) {
         if (jp == X.p) continue;
-        const float4 o = __ldg(&sp[jp]);
-        float ex = X.me.x - o.x, ey = X.me.y - o.y, ez = (D == 3) ? X.me.z - o.z : 0.f;
+        const float4 o = __ldg(&V.sp[jp]);
+        float ex = mx - o.x, ey = my - o.y, ez = (D == 3) ? X.z - o.z : 0.f;
         if (ex == 0.f && ey == 0.f && (D == 2 || ez == 0.f)) {
-            const uint32_t oj = __ldg(&V.sorig[jp]);
-            const float sg = X.oi < oj ? 1.f : -1.f;
-            ex = sg * (float)jiggle(V.seed, iter, 0, X.oi, oj);
-            ey = sg * (float)jiggle(V.seed, iter, 1, X.oi, oj);
-            if (D == 3) ez = sg * (float)jiggle(V.seed, iter, 2, X.oi, oj);
+            const uint32_t oi = __ldg(&V.sorig[X.p]), oj = __ldg(&V.sorig[jp]);
+            const float sg = oi < oj ? 1.f : -1.f;
+            ex = sg * (float)jiggle(V.seed, V.iter, 0, oi, oj);
+            ey = sg * (float)jiggle(V.seed, V.iter, 1, oi, oj);
+            if (D == 3) ez = sg * (float)jiggle(V.seed, V.iter, 2, oi, oj);
         }
-        const float e2 = (D == 3) ? ex * ex + ey * ey + ez * ez : ex * ex + ey * ey;
+        float e2 = __fmaf_rn(ex, ex, __fmul_rn(ey, ey));
+        if (D == 3) e2 = __fmaf_rn(ez, ez, e2);
         const float g = __fdividef(X.mk * o.w, e2);
-        X.f0 += ex * g;
-        X.f1 += ey * g;
-        if (D == 3) X.f2 += ez * g;
-        if (COUNT) X.npair++;
+        X.f0 = __fmaf_rn(ex, g, X.f0);
+        X.f1 = __fmaf_rn(ey, g, X.f1);
+        if (D == 3) X.f2_ = __fmaf_rn(ez, g, X.f2_);
+        X.npair++;
     }
 }
 
-// Two adjacent Morton-sorted nodes per thread over the union of their walks:
-// one cell load and one loop step serve both, and each node acts only at the
-// cells of its own walk (k >= its resume), in the same order, so its forces are
-// walk_lane's bit for bit. Adjacent nodes' walks nearly coincide, so the union
-// is little longer than either.
-template <int D, bool COUNT = true>
-__device__ __forceinline__ void walk_pair(const WalkView &V, PairNode &a, PairNode &b) {
-    const Cells cells = V.cells;
-    const uint32_t ncells = V.ncells;
-    uint32_t k = min(a.resume, b.resume);
-    while (k < ncells) {
-        const float4 A = cell_a<D>(cells, k);
-        const float4 B = cell_b<D>(cells, k);
-        int32_t sk;
-        uint32_t start;
-        float cx, cy, cz, cm, w2, lx, ly, lz;
-        if (D == 2) {
-            cx = A.x; cy = A.y; cz = 0.f; cm = A.z; w2 = A.w;
-            lx = B.x; ly = B.y; lz = 0.f;
-            sk = __float_as_int(B.z);
-            start = __float_as_uint(B.w);
-        } else {
-            const int2 Cc = cell_c3(cells, k);
-            cx = A.x; cy = A.y; cz = A.z; cm = A.w;
-            lx = B.x; ly = B.y; lz = B.z; w2 = B.w;
-            sk = Cc.x;
-            start = (uint32_t)Cc.y;
+// The visit of cell k, its records R, by a node (act: when it takes part in it):
+// a body term (a far cell, or a leaf of one point at any distance) is added.
+// Returns whether it was, so that the node leaves the subtree out. All of it is
+// selected, not branched: the term is added as +-0 when it does not count (an
+// exact no-op: the sums start at +0 and never hold -0). d2 is at least 2^-108
+// where it counts: points in different leaves have different keys, so on some
+// axis their FP64 offsets from the root's corner (an integer) differ across a
+// multiple of 2^-32 of its side (>= 1), which FP32 coordinates nearer than 2^-54
+// to each other never do.
+template <int D, bool COUNT>
+__device__ __forceinline__ bool node_body(const WalkView &V, WalkNode &X, const CellRec<D> &R, uint32_t k, bool act) {
+    const bool holds = k <= X.mylp && X.mylp < R.skip;
+    float dx, dy, dz, d2;
+    cell_offset<D>(R, X.xy, X.z, dx, dy, dz, d2);
+    const float t = V.th2 * d2;
+    const bool body = act && !holds && R.w2 < t;  // w2 < 0 (one point): always, w2 > 0: far
+    const float fb = __fmul_rn(X.mk * R.m, rcp_ftz(d2));
+    const float f = body ? fb : 0.f;
+    X.f0 = __fmaf_rn(dx, f, X.f0);
+    X.f1 = __fmaf_rn(dy, f, X.f1);
+    if (D == 3) X.f2_ = __fmaf_rn(dz, f, X.f2_);
+    if (COUNT) {  // a one-point leaf too near to be far is an exact pair
+        const bool far = body && fabsf(R.w2) < t;
+        X.nfar += far ? 1u : 0u;
+        X.npair += body && !far ? 1u : 0u;
+    }
+    return body;
+}
+
+// A leaf of several points that is not far: its points one by one.
+template <int D>
+__device__ __forceinline__ void node_multi(const WalkView &V, WalkNode &X, uint32_t k) {
+    node_pairs<D>(V, X, __ldg(&V.cells.range[k]));
+}
+
+template <int D, bool COUNT>
+__device__ __forceinline__ bool node_visit(const WalkView &V, WalkNode &X, const CellRec<D> &R, uint32_t k) {
+    const bool body = node_body<D, COUNT>(V, X, R, k, true);
+    if (!body && R.multi) node_multi<D>(V, X, k);
+    return body;
+}
+
+// One cell of a node's own walk (X.k < ncells). Every step moves forward,
+// whatever a cell holds.
+template <int D, bool COUNT>
+__device__ __forceinline__ void node_step(const WalkView &V, WalkNode &X, const CellRec<D> &R) {
+    const uint32_t k = X.k;
+    const bool body = node_visit<D, COUNT>(V, X, R, k);
+    X.k = body ? max(R.skip, k + 1) : k + 1;
+}
+
+// Per-lane walk: every lane on its own cell index (gathered cell loads, no warp
+// vote), so the warp runs as long as its longest path.
+template <int D, bool COUNT, bool WIDE>
+__device__ __forceinline__ void walk_own(const WalkView &V, WalkNode &X) {
+    while (X.k < V.ncells) node_step<D, COUNT>(V, X, cell_rec<D, WIDE>(V.cells, X.k));
+}
+
+// Union walk of a warp: the cell index is the same in every lane (one broadcast
+// load); each lane keeps in X.k the first cell it takes part in again after it
+// left a subtree out. The warp descends when any lane opens the cell and jumps
+// to skip otherwise; a lane acts only at the cells of its own walk.
+template <int D, bool COUNT>
+__device__ __forceinline__ void walk_group(const WalkView &V, WalkNode &X) {
+    uint32_t k = 0;
+    while (k < V.ncells) {
+        const CellRec<D> R = cell_rec<D, false>(V.cells, k);
+        const uint32_t skip = max(R.skip, k + 1);
+        bool open = false;
+        if (X.k <= k) {
+            open = !node_visit<D, COUNT>(V, X, R, k);
+            X.k = open ? k + 1 : skip;
         }
-        const bool leaf = sk < 0;
-        // leaves move on to k + 1; every step moves forward, whatever a cell holds
-        const uint32_t skip = (uint32_t)max(sk, (int32_t)k + 1);
-        pair_visit<D, COUNT>(V, a, k, cx, cy, cz, lx, ly, lz, cm, w2, sk, start, skip, leaf);
-        pair_visit<D, COUNT>(V, b, k, cx, cy, cz, lx, ly, lz, cm, w2, sk, start, skip, leaf);
-        k = min(a.resume, b.resume);
+        __syncwarp();
+        k = __any_sync(GR_FULL, open) ? k + 1 : skip;
     }
 }
 
-// Two independent per-lane walks per thread, stepped in turn: the lane's nodes
-// p and p + 32 (a warp holds two groups of 32 consecutive sorted nodes, each
-// group as coherent as walk_lane's warp), each with its own cell index. Both
-// walks' cell records are requested before either is used, so every thread
-// keeps two dependent chains of cell loads in flight where walk_lane keeps
-// one. A walk that has finished re-reads its last cell (a cached load) and
-// does nothing with it. Each node visits its own cells in its own order with
-// lane_visit's arithmetic, so its forces are walk_lane's bit for bit.
-template <int D, bool COUNT = true>
-__device__ __forceinline__ void walk_two(const WalkView &V, LaneNode &a, LaneNode &b) {
-    const uint32_t nc = V.ncells;
-    const uint32_t last = nc - 1u;  // nc >= 1 whenever a node is valid
-    while (a.k < nc || b.k < nc) {
-        const CellRec ra = cell_rec<D>(V.cells, min(a.k, last));
-        const CellRec rb = cell_rec<D>(V.cells, min(b.k, last));
-        if (a.k < nc) lane_visit<D, COUNT>(V, a, ra);
-        if (b.k < nc) lane_visit<D, COUNT>(V, b, rb);
+// N adjacent Morton-sorted nodes per thread over the union of their walks: one
+// cell load and one loop step serve all of them, and each node acts only at the
+// cells of its own walk (k >= its X.k), in the same order, so its forces are
+// the per-lane walk's bit for bit. Adjacent nodes' walks nearly coincide, so the
+// union is little longer than one.
+template <int D, int N, bool COUNT, bool WIDE>
+__device__ __forceinline__ void walk_union(const WalkView &V, WalkNode *X) {
+    uint32_t k = X[0].k;  // the first node is valid whenever any is
+    while (k < V.ncells) {
+        const CellRec<D> R = cell_rec<D, WIDE>(V.cells, k);
+        const uint32_t skip = max(R.skip, k + 1);
+        uint32_t next = 0xffffffffu, open = 0u;
+#pragma unroll
+        for (int j = 0; j < N; j++) {
+            const bool act = X[j].k <= k;
+            const bool body = node_body<D, COUNT>(V, X[j], R, k, act);
+            if (act && !body) open |= 1u << j;
+            X[j].k = body ? skip : act ? k + 1 : X[j].k;
+            next = min(next, X[j].k);
+        }
+        if (open && R.multi) {
+#pragma unroll
+            for (int j = 0; j < N; j++)
+                if (open >> j & 1u) node_multi<D>(V, X[j], k);
+        }
+        k = next;
     }
 }
 
 // Walk schedules: 0 = walk_group (a warp over the union of its 32 nodes),
-// 1 = walk_lane (one node per lane), 2 = walk_pair (two adjacent nodes per
-// lane), 3 = walk_two (two independent walks per lane, 32 nodes apart).
+// 1 = one node per lane, 2 and 3 = walk_union (two or four adjacent nodes per
+// lane).
 // COUNT: add the far / pair interaction counts to the state (a diagnostic; the
-// forces are the same either way).
-template <int D, int SCHED, bool COUNT>
-__global__ void __launch_bounds__(WALK_THREADS)
+// forces are the same either way). WIDE: the tree keeps skip in an array of its
+// own (one or two nodes per lane only).
+
+// Nodes a lane, and the resident blocks of 256 threads per SM the registers are
+// budgeted for, the fastest at 1M nodes (walk beside the attraction, us). 2D: one
+// node a lane 193 / 193 / 184 / 183 at 5 .. 8 blocks, two 197 / 196 / 199 / 187 at
+// 3 .. 6, four 213 / 202 / 211 at 3 .. 5; 3D: one 418 / 411 / 410 / 411 at 5 .. 8,
+// two 343 / 340 / 325 / 370 at 3 .. 6, four 343 / 340 / 484 at 3 .. 5.
+template <int D, int SCHED>
+struct WalkOcc {
+    static constexpr int N = SCHED == 3 ? 4 : SCHED == 2 ? 2 : 1;
+    static constexpr int MIN_BLOCKS = SCHED == 3 ? 4 : SCHED == 2 ? (D == 3 ? 5 : 6) : D == 3 ? 7 : 8;
+};
+
+template <int D, int SCHED, bool COUNT, bool WIDE>
+__global__ void __launch_bounds__(WALK_THREADS, WalkOcc<D, SCHED>::MIN_BLOCKS)
 k_walk_s(WalkParams P, const DevState *__restrict__ st, Cells cells, const float4 *__restrict__ sp,
          const uint32_t *__restrict__ sorig, const uint32_t *__restrict__ uid,
          const uint32_t *__restrict__ leaf_pre, float *__restrict__ rep, DevState *stw) {
@@ -468,59 +275,36 @@ k_walk_s(WalkParams P, const DevState *__restrict__ st, Cells cells, const float
     if (st->converged) return;
     const uint32_t g = blockIdx.x * WALK_THREADS + threadIdx.x;
     const uint32_t lane = threadIdx.x % GR_WARP;
-    const uint32_t p = SCHED == 2 ? 2 * g : SCHED == 3 ? 2 * (g - lane) + lane : g;
+    constexpr int N = WalkOcc<D, SCHED>::N;
+    const uint32_t p = N * g;
     if (__all_sync(GR_FULL, p >= P.n)) return;
-    WalkView V{cells, sp, sorig, uid, leaf_pre, P.n, st->n_cells, st->iter_no, P.seed, P.kr, P.theta2, &stw->error};
-    uint32_t nfar, npair;
-    if (SCHED == 3) {
-        LaneNode a, b;
-        lane_init<D>(V, p, a);
-        lane_init<D>(V, p + GR_WARP, b);
-        walk_two<D, COUNT>(V, a, b);
-        const LaneNode *X[2] = {&a, &b};
+    const WalkView V{cells, sp, sorig, uid, leaf_pre, P.n, st->n_cells, st->iter_no, P.seed, P.kr, P.theta2,
+                     &stw->error};
+    WalkNode X[N];
 #pragma unroll
-        for (int j = 0; j < 2; j++)
-            if (X[j]->p < P.n) {
-                const uint32_t oi = X[j]->oi;
-                rep[(size_t)oi * D + 0] = X[j]->f0;
-                rep[(size_t)oi * D + 1] = X[j]->f1;
-                if (D == 3) rep[(size_t)oi * D + 2] = X[j]->f2;
-            }
-        nfar = a.nfar + b.nfar;
-        npair = a.npair + b.npair;
-    } else if (SCHED == 2) {
-        PairNode a, b;
-        pair_init<D>(V, p, a);
-        pair_init<D>(V, p + 1, b);
-        walk_pair<D, COUNT>(V, a, b);
-        const PairNode *X[2] = {&a, &b};
+    for (int j = 0; j < N; j++) node_init<D>(V, p + j, X[j]);
+    if (N > 1)
+        walk_union<D, N, COUNT, WIDE>(V, X);
+    else if (SCHED == 1)
+        walk_own<D, COUNT, WIDE>(V, X[0]);
+    else
+        walk_group<D, COUNT>(V, X[0]);
+    uint32_t nfar = 0, npair = 0;
 #pragma unroll
-        for (int j = 0; j < 2; j++)
-            if (X[j]->p < P.n) {
-                const uint32_t oi = X[j]->oi;
-                rep[(size_t)oi * D + 0] = X[j]->f0;
-                rep[(size_t)oi * D + 1] = X[j]->f1;
-                if (D == 3) rep[(size_t)oi * D + 2] = X[j]->f2;
-            }
-        nfar = a.nfar + b.nfar;
-        npair = a.npair + b.npair;
-    } else {
-        float f0, f1, f2;
-        if (SCHED == 1)
-            walk_lane<D, COUNT>(V, p, f0, f1, f2, nfar, npair);
-        else
-            walk_group<D, COUNT>(V, p, f0, f1, f2, nfar, npair);
-        if (p < P.n) {
-            const uint32_t oi = sorig[p];
-            rep[(size_t)oi * D + 0] = f0;
-            rep[(size_t)oi * D + 1] = f1;
-            if (D == 3) rep[(size_t)oi * D + 2] = f2;
+    for (int j = 0; j < N; j++) {
+        if (X[j].p < P.n) {
+            const uint32_t oi = sorig[X[j].p];
+            rep[(size_t)oi * D + 0] = X[j].f0;
+            rep[(size_t)oi * D + 1] = X[j].f1;
+            if (D == 3) rep[(size_t)oi * D + 2] = X[j].f2_;
         }
+        nfar += X[j].nfar;
+        npair += X[j].npair;
     }
     if (!COUNT) return;
     nfar = __reduce_add_sync(GR_FULL, nfar);
     npair = __reduce_add_sync(GR_FULL, npair);
-    if ((threadIdx.x % GR_WARP) == 0) {
+    if (lane == 0) {
         atomicAdd(&stw->far_count, (unsigned long long)nfar);
         atomicAdd(&stw->pair_count, (unsigned long long)npair);
     }

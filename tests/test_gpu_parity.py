@@ -126,6 +126,20 @@ def test_forces_past_the_one_pass_scan_limit():
     assert abs(info["far_count"] - sc["far"]) <= 1e-3 * sc["far"]
 
 
+@pytest.mark.parametrize("n,dim", [(2_097_151, 2), (2_097_152, 2), (2_097_152, 3)])
+def test_forces_either_side_of_the_cell_records_skip(n, dim):
+    """Past 2^21 - 1 nodes a tree's skips leave the 22 bits of its cell records for an array of their
+    own. Every schedule gives the same forces; they match the oracle to the file's tolerance."""
+    wl = synth.powerlaw_1m(n=n, dim=dim)
+    with Fa2(wl.n, wl.src, wl.dst, params=wl.params, pos0=wl.pos0) as eng:
+        ref = eng.forces()
+        for sch in (0, 1, 2, 3):
+            eng.set_walk_schedule(sch)
+            assert np.array_equal(eng.forces(), ref)
+    st = oracle_state(wl.n, wl.src, wl.dst, None, wl.pos0, wl.params)
+    assert rel_l2(ref.astype(np.float64), st.accumulate(7)) < TOL
+
+
 def test_run_is_deterministic():
     wl = synth.sbm_1500()
     outs = []
