@@ -23,6 +23,7 @@
 #include "common.cuh"
 #include "forces.cuh"
 #include "tree.cuh"
+#include "walk.cuh"
 
 namespace gr {
 
@@ -49,13 +50,12 @@ __device__ __forceinline__ double d3_cool(double alpha, double target, double de
     return __dadd_rn(alpha, __dmul_rn(__dsub_rn(target, alpha), decay));
 }
 
-// Projected records {x + vx, y + vy, degree, 1}: the link's state (link.rs
-// displaced). The degree rides along so that the link pass reads a neighbour in
-// one 16-byte load. Thread 0 also advances the cooling schedule and the tick
+// Projected records {x + vx, y + vy, 0, 1}: the link's state (link.rs displaced).
+// Thread 0 also advances the cooling schedule and the tick
 // count, which nothing else in this kernel reads; the tick's later kernels key
 // their jiggles on tick_no - 1.
 __global__ void k_d3_project(uint32_t n, const float4 *__restrict__ p, const float2 *__restrict__ v,
-                             const uint32_t *__restrict__ rp, float4 *__restrict__ pp, D3State *s, double decay) {
+                             float4 *__restrict__ pp, D3State *s, double decay) {
     const uint32_t i = blockIdx.x * D3_T + threadIdx.x;
     if (i == 0) {
         s->alpha = d3_cool(s->alpha, s->alpha_target, decay);
@@ -64,7 +64,7 @@ __global__ void k_d3_project(uint32_t n, const float4 *__restrict__ p, const flo
     if (i >= n) return;
     const float4 a = p[i];
     const float2 b = v[i];
-    pp[i] = make_float4(a.x + b.x, a.y + b.y, (float)(rp[i + 1] - rp[i]), 1.f);
+    pp[i] = make_float4(a.x + b.x, a.y + b.y, 0.f, 1.f);
 }
 
 // One directed CSR entry of the link pass, laid out once per session: the
@@ -74,7 +74,8 @@ __global__ void k_d3_project(uint32_t n, const float4 *__restrict__ p, const flo
 // Per tick that leaves a node one square root and one division an entry; with
 // the degrees, the rest length and the share worked out every tick (two divisions
 // and two random reads of row offsets an entry more) the pass took 112 us at 1M
-// nodes and 3.1M entries, with the table 67 us.
+// nodes and 3.1M entries, with the table 79, with the terms spread over the warp
+// as well (forces.cuh) 43.
 struct D3Link {
     uint32_t u;
     float dist, str, share;
@@ -100,79 +101,38 @@ __global__ void k_d3_link_table(D3Params P, uint32_t n, const uint32_t *__restri
                    v == b ? -bias : 1.f - bias};
 }
 
-// Node v's share of one simple edge (link.rs force + share); me = pp[v].
-__device__ __forceinline__ void d3_link_term(const D3Params &P, uint32_t v, const float4 &me, const D3Link &k,
-                                             float alpha, uint32_t tick, const float4 *__restrict__ pp, float &ax,
-                                             float &ay) {
-    const float4 o = pp[k.u];
-    const bool high = v > k.u;  // the displacement runs from the lower node to the higher
-    float dx = high ? me.x - o.x : o.x - me.x, dy = high ? me.y - o.y : o.y - me.y;
-    if (dx == 0.f || dy == 0.f) {
-        const uint32_t lo = min(k.u, v), hi = max(k.u, v);
-        if (dx == 0.f) dx = (float)jiggle(P.seed, tick, 0, lo, hi);
-        if (dy == 0.f) dy = (float)jiggle(P.seed, tick, 1, lo, hi);
-    }
-    const float l = sqrtf(dx * dx + dy * dy);
-    if (l == 0.f) return;
-    const float factor = (l - k.dist) / l * alpha * k.str;
-    ax += dx * factor * k.share;
-    ay += dy * factor * k.share;
-}
-
-__device__ __forceinline__ D3Link d3_link_load(const D3Link *__restrict__ lk, uint32_t e) {
-    const uint4 q = __ldg((const uint4 *)lk + e);
-    return D3Link{q.x, __uint_as_float(q.y), __uint_as_float(q.z), __uint_as_float(q.w)};
-}
-
-// Heavy rows: one warp per SEG-entry segment, summed by a fixed butterfly.
-__global__ void __launch_bounds__(D3_T)
-k_d3_link_seg(D3Params P, uint32_t nseg, const D3State *st, const float4 *__restrict__ pp,
-              const uint32_t *__restrict__ rp, const D3Link *__restrict__ lk, const uint32_t *__restrict__ seg_row,
-              const uint32_t *__restrict__ seg_first, float2 *__restrict__ seg_out) {
-    const uint32_t sg = (blockIdx.x * D3_T + threadIdx.x) / GR_WARP, lane = threadIdx.x % GR_WARP;
-    if (sg >= nseg) return;
-    const uint32_t row = seg_row[sg];
-    const uint32_t e0 = rp[row] + (sg - seg_first[row]) * SEG, e1 = min(e0 + SEG, rp[row + 1]);
-    const float alpha = (float)st->alpha;
-    float ax = 0.f, ay = 0.f;
-    const uint32_t tick = st->tick_no - 1u;
-    const float4 me = pp[row];
-    for (uint32_t e = e0 + lane; e < e1; e += GR_WARP)
-        d3_link_term(P, row, me, d3_link_load(lk, e), alpha, tick, pp, ax, ay);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        ax += __shfl_xor_sync(GR_FULL, ax, o);
-        ay += __shfl_xor_sync(GR_FULL, ay, o);
-    }
-    if (lane == 0) seg_out[sg] = make_float2(ax, ay);
-}
-
-// Every node's link delta (its row in CSR order; heavy rows from their
-// segments in order) onto its own velocity. Reads only the projected records.
-__global__ void __launch_bounds__(D3_T)
+// Every node's link delta (its row in CSR order) onto its own velocity. Reads
+// only the projected records. An entry's term is its correction along the edge
+// times the row's share (link.rs force + share).
+__global__ void __launch_bounds__(FRC_THREADS)
 k_d3_link(D3Params P, const D3State *st, const float4 *__restrict__ pp, const uint32_t *__restrict__ rp,
-          const D3Link *__restrict__ lk, const uint32_t *__restrict__ seg_first, const float2 *__restrict__ seg_out,
-          float2 *__restrict__ v) {
-    const uint32_t i = blockIdx.x * D3_T + threadIdx.x;
-    if (i >= P.n) return;
+          const D3Link *__restrict__ lk, Segments G, float2 *__restrict__ v) {
     const float alpha = (float)st->alpha;
-    const uint32_t e0 = rp[i], e1 = rp[i + 1];
-    float ax = 0.f, ay = 0.f;
-    if (seg_first == nullptr || e1 - e0 <= LIGHT_MAX) {
-        const uint32_t tick = st->tick_no - 1u;
-        const float4 me = pp[i];
-        for (uint32_t e = e0; e < e1; e++) d3_link_term(P, i, me, d3_link_load(lk, e), alpha, tick, pp, ax, ay);
-    } else {
-        const uint32_t s0 = seg_first[i], ns = (e1 - e0 + SEG - 1) / SEG;
-        for (uint32_t s = s0; s < s0 + ns; s++) {
-            ax += seg_out[s].x;
-            ay += seg_out[s].y;
-        }
-    }
-    float2 w = v[i];
-    w.x += ax;
-    w.y += ay;
-    v[i] = w;
+    const uint32_t tick = st->tick_no - 1u;
+    block_rows<2>(
+        P.n, pp, rp, G, [&](uint32_t e) { return __ldg(&lk[e].u); },
+        [&](const float4 &me, uint32_t i, uint32_t e, const float4 &o, float *d) {
+            const uint4 q = __ldg((const uint4 *)lk + e);
+            const D3Link k{q.x, __uint_as_float(q.y), __uint_as_float(q.z), __uint_as_float(q.w)};
+            const bool high = i > k.u;  // the displacement runs from the lower node to the higher
+            float dx = high ? me.x - o.x : o.x - me.x, dy = high ? me.y - o.y : o.y - me.y;
+            if (dx == 0.f || dy == 0.f) {
+                const uint32_t lo = min(k.u, i), hi = max(k.u, i);
+                if (dx == 0.f) dx = (float)jiggle(P.seed, tick, 0, lo, hi);
+                if (dy == 0.f) dy = (float)jiggle(P.seed, tick, 1, lo, hi);
+            }
+            const float l = sqrtf(dx * dx + dy * dy);
+            const float factor = l == 0.f ? 0.f : (l - k.dist) / l * alpha * k.str;
+            d[0] = __fmul_rn(dx, factor);
+            d[1] = __fmul_rn(dy, factor);
+            return k.share;
+        },
+        [&](uint32_t i, const float *acc) {
+            float2 w = v[i];
+            w.x += acc[0];
+            w.y += acc[1];
+            v[i] = w;
+        });
 }
 
 // charge.rs settle: false past distanceMax; a zero axis jiggled (passes 2, 3);
@@ -193,14 +153,26 @@ __device__ __forceinline__ bool d3_settle(const D3Params &P, uint32_t tick, uint
     return true;
 }
 
+constexpr int D3_LIST = 20;  // cells or points a lane lists at a time
+
 // Many-body: per sorted node, the stackless preorder walk of charge.rs
-// node_delta over the cells (their mass is their point count); the delta goes onto the node's own velocity. A cell the
-// opening test resolves acts as one body of its count; a leaf it does not takes
-// its points directly, every point at the leaf centre's offset (charge.rs
-// direct), which is the same term with the count less this node when it lies in
-// the leaf. So the common outcomes need no branch: the term is selected by
-// predicate, the next cell by select; only an exactly zero axis (the jiggle)
-// branches.
+// node_delta over the cells (their mass is their point count); the delta goes
+// onto the node's own velocity. A cell the opening test resolves acts as one body
+// of its count; a leaf it does not takes its points directly, every point at the
+// leaf centre's offset (charge.rs direct), which is the same term with the count
+// less this node when it lies in the leaf.
+//
+// Bound by instruction issue. The common outcomes need no branch (the term is
+// selected, the next cell too); a leaf of several points, a centre nearer than
+// distanceMin and an exactly zero axis (the jiggle) branch off together. A node
+// meets itself at zero on both axes, each lane of a warp at another step, so its
+// own leaf must not take the jiggle's branch: 421 us at 1M nodes with it (376M warp
+// instructions, half of the lanes' slots in it idle), 360 without (309M).
+// Measured with it and left out: a lane listing
+// the cells that count and the warp taking the lists' terms together (492), the
+// term in a branch of its own with subtrees past distanceMax left out by their
+// squares (512; 15% fewer steps).
+template <bool WIDE>
 __global__ void __launch_bounds__(D3_T)
 k_d3_charge(D3Params P, const D3State *st, const DevState *ts, Cells cells, const float4 *__restrict__ sp,
             const uint32_t *__restrict__ sorig, float2 *__restrict__ v) {
@@ -209,47 +181,48 @@ k_d3_charge(D3Params P, const D3State *st, const DevState *ts, Cells cells, cons
     const uint32_t ncells = ts->n_cells, tick = st->tick_no - 1u;
     const float ca = P.charge * (float)st->alpha;
     const float4 me = sp[p];
-    const uint32_t oi = sorig[p];
+    const f2 xy = f2_pack(me.x, me.y);
     float ax = 0.f, ay = 0.f;
     uint32_t k = 0;
     while (k < ncells) {
-        CellRec<2> R = cell_rec<2, false>(cells, k);
-        if (cells.skip) R.skip = __ldg(&cells.skip[k]);
-        const bool multi = R.multi, leaf = multi || R.w2 < 0.f;
-        // the displacement to the centre: the records hold it negated
-        float dx = -((me.x + R.a.x) + R.lx), dy = -((me.y + R.a.y) + R.ly);
-        float l = dx * dx + dy * dy;
-        const bool open = fabsf(R.w2) >= P.th2 * l;  // open >= l: w^2 / theta^2 >= l
-        const bool in_range = l < P.dmax2;           // settle: nothing at or past distanceMax
-        bool self_in = false;  // this node is one of the leaf's points
-        if (multi || dx == 0.f || dy == 0.f) {  // this node is in no other leaf
-            const uint32_t start = __ldg(&cells.start[k]), last = multi ? __ldg(&cells.range[k].y) - 1u : start;
-            self_in = leaf && p >= start && p <= last;
-            // the jiggle, keyed on the chain head (direct) or the cell (body)
-            const uint32_t key = (open && leaf) ? __ldg(&sorig[last]) : k;
-            if (dx == 0.f) {
-                dx = (float)jiggle(P.seed, tick, 2, oi, key);
-                l += dx * dx;
-            }
-            if (dy == 0.f) {
-                dy = (float)jiggle(P.seed, tick, 3, oi, key);
-                l += dy * dy;
-            }
-        }
-        l = l < P.dmin2 ? sqrtf(P.dmin2 * l) : l;
-        l = l == 0.f ? fmaxf(P.dmin2, 1.17549435e-38f) : l;
+        const CellRec<2> R = cell_rec<2, WIDE>(cells, k);
+        // the records hold the centre negated: minus the displacement to it
+        float nx, ny, nz, l;
+        cell_offset<2>(R, xy, 0.f, nx, ny, nz, l);
+        const float w2 = fabsf(R.w2);
+        const bool leaf = R.multi || R.w2 < 0.f, open = w2 >= P.th2 * l;  // open >= l: w^2 / theta^2 >= l
         const bool descend = open && !leaf;
-        const bool counted = !descend && in_range;
-        const float m = (open && self_in) ? R.m - 1.f : R.m;
-        const float f = counted ? m * ca / l : 0.f;
-        ax += dx * f;
-        ay += dy * f;
+        // settle: nothing at or past distanceMax. The leaf of this node alone has no
+        // other point (its term is 0, whatever its jiggle): no other leaf of one
+        // point has its coordinates
+        const bool counted = !descend && l < P.dmax2 && !(R.w2 < 0.f && l == 0.f);
+        float m = R.m;
+        if (counted && (R.multi || l < P.dmin2 || fminf(fabsf(nx), fabsf(ny)) == 0.f)) {
+            const uint32_t start = __ldg(&cells.start[k]), last = R.multi ? __ldg(&cells.range[k].y) - 1u : start;
+            if (open && leaf && p >= start && p <= last) m -= 1.f;  // this node is one of the leaf's points
+            // the jiggle, keyed on the chain head (direct) or the cell (body)
+            const uint32_t oi = sorig[p], key = (open && leaf) ? __ldg(&sorig[last]) : k;
+            if (nx == 0.f) {
+                nx = -(float)jiggle(P.seed, tick, 2, oi, key);
+                l += nx * nx;
+            }
+            if (ny == 0.f) {
+                ny = -(float)jiggle(P.seed, tick, 3, oi, key);
+                l += ny * ny;
+            }
+            l = l < P.dmin2 ? sqrtf(P.dmin2 * l) : l;
+            l = l == 0.f ? fmaxf(P.dmin2, 1.17549435e-38f) : l;
+        }
+        const float q = m * ca / (counted ? l : 1.f), f = counted ? q : 0.f;  // never a quotient by 0
+        ax = __fmaf_rn(-nx, f, ax);
+        ay = __fmaf_rn(-ny, f, ay);
         k = descend ? k + 1 : max(R.skip, k + 1);
     }
-    float2 w = v[oi];
-    w.x += ax;
-    w.y += ay;
-    v[oi] = w;
+    const uint32_t oi = sorig[p];
+    float2 u = v[oi];
+    u.x += ax;
+    u.y += ay;
+    v[oi] = u;
 }
 
 // ---- collide: every other point within reach = 2 r of the projected position
@@ -261,7 +234,7 @@ k_d3_charge(D3Params P, const D3State *st, const DevState *ts, Cells cells, cons
 // order as a walk of the quadtree's leaves, bit for bit. That quadtree and its
 // walk stood here before: at 1M nodes the leaf pass, the radix tree, the scan,
 // the cell writer and the walk took 595 us of the tick, the gather and the scan
-// of the cells take 290 us.
+// of the cells take 205 us.
 //
 // The runs are found in a table of one entry a cell, as many entries as nodes or
 // more. A drawing whose box needs a deeper level than the table holds
@@ -395,14 +368,16 @@ k_d3_collide(D3Params P, const D3State *st, const DevState *ts, const D3Grid *gr
              const float4 *__restrict__ sp, const uint2 *__restrict__ table, float4 *__restrict__ pos,
              float2 *__restrict__ v) {
     gr_pdl_enter();
+    __shared__ uint32_t s_list[D3_LIST][D3_T];
     const uint32_t p = blockIdx.x * D3_T + threadIdx.x;
-    if (p >= P.n || ts->converged) return;
+    if (ts->converged || (p & ~(GR_WARP - 1u)) >= P.n) return;  // whole warps only
+    const bool valid = p < P.n;
     const uint32_t tick = st->tick_no - 1u;
     const int level = grid->level, deeper = 2 * (level - grid->table_level), shift = 64 - 2 * level;
-    const float4 q = sp[p];
+    const float4 q = sp[valid ? p : P.n - 1];
     const uint32_t oi = __float_as_uint(q.z);
     // the cell's coordinates from its Morton index, and its neighbours' runs
-    const uint64_t cell = keys[p] >> shift;
+    const uint64_t cell = keys[valid ? p : P.n - 1] >> shift;
     const uint32_t cx = compact2(cell), cy = compact2(cell >> 1), top = (1u << level) - 1u;
     uint32_t lo[9], hi[9];
 #pragma unroll
@@ -410,7 +385,7 @@ k_d3_collide(D3Params P, const D3State *st, const DevState *ts, const D3Grid *gr
         const uint32_t x = cx + (uint32_t)(r % 3) - 1u, y = cy + (uint32_t)(r / 3) - 1u;
         lo[r] = 0xffffffffu;  // no points: sorts last
         hi[r] = 0u;
-        if (x > top || y > top || !(P.reach2 > 0.f)) continue;
+        if (!valid || x > top || y > top || !(P.reach2 > 0.f)) continue;
         const uint64_t c = spread2(x) | (spread2(y) << 1);
         uint2 e = __ldg(&table[c >> deeper]);
         if (deeper && e.x < e.y) {
@@ -434,29 +409,56 @@ k_d3_collide(D3Params P, const D3State *st, const DevState *ts, const D3Grid *gr
             hi[b - 1] = h0;
             hi[b] = h1;
         }
+    // the points in reach, in order, listed first and pushed afterwards: the square
+    // root and the quotient then run for as many rounds as the warp's longest list,
+    // not for every round in which any lane finds a point
     float ax = 0.f, ay = 0.f;
-#pragma unroll
-    for (int r = 0; r < 9; r++)
-        for (uint32_t j = lo[r]; j < hi[r]; j++) {
-            if (j == p) continue;
+    uint32_t found = 0;
+    auto push = [&]() {
+        for (uint32_t f = 0; f < found; f++) {
+            const uint32_t j = s_list[f][threadIdx.x];
             const float4 o = __ldg(&sp[j]);
             float dx = q.x - o.x, dy = q.y - o.y;
             float l = dx * dx + dy * dy;
-            if (l >= P.reach2) continue;
-            const uint32_t oj = __float_as_uint(o.z);
-            if (dx == 0.f) {
-                dx = (float)jiggle(P.seed, tick, 4, oi, oj);
-                l += dx * dx;
-            }
-            if (dy == 0.f) {
-                dy = (float)jiggle(P.seed, tick, 5, oi, oj);
-                l += dy * dy;
+            if (dx == 0.f || dy == 0.f) {
+                const uint32_t oj = __float_as_uint(o.z);
+                if (dx == 0.f) {
+                    dx = (float)jiggle(P.seed, tick, 4, oi, oj);
+                    l += dx * dx;
+                }
+                if (dy == 0.f) {
+                    dy = (float)jiggle(P.seed, tick, 5, oi, oj);
+                    l += dy * dy;
+                }
             }
             const float dist = sqrtf(l);
-            const float push = (P.reach - dist) / dist * 0.5f;
-            ax += dx * push;
-            ay += dy * push;
+            const float amount = (P.reach - dist) / dist * 0.5f;
+            ax += dx * amount;
+            ay += dy * amount;
         }
+        found = 0;
+    };
+#pragma unroll
+    for (int r = 0; r < 9; r++) {
+        const uint32_t rounds = __reduce_max_sync(GR_FULL, lo[r] < hi[r] ? (hi[r] - lo[r] + 3) / 4 : 0u);
+        for (uint32_t k = 0; k < rounds; k++) {
+            const uint32_t j0 = lo[r] + 4 * k;
+            if (lo[r] < hi[r] && j0 < hi[r]) {
+                float4 o[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) o[u] = __ldg(&sp[min(j0 + u, hi[r] - 1)]);
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const float dx = q.x - o[u].x, dy = q.y - o[u].y;
+                    const float l = dx * dx + dy * dy;
+                    if (j0 + u < hi[r] && j0 + u != p && !(l >= P.reach2)) s_list[found++][threadIdx.x] = j0 + u;
+                }
+            }
+            if (__any_sync(GR_FULL, found > D3_LIST - 4)) push();  // together: the lanes fill at about the same rate
+        }
+    }
+    push();
+    if (!valid) return;
     float2 w = v[oi];
     w.x += ax;
     w.y += ay;

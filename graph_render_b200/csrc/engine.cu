@@ -140,6 +140,7 @@ struct gr_fa2 {
     uint32_t *seg_row = nullptr;       // segment -> row
     uint32_t *seg_first = nullptr;     // row -> its first segment (heavy rows)
     float *seg_out = nullptr;          // segment sums, D per segment
+    uint32_t *seg_done = nullptr;      // a row's finished segments, at its first one (0 between launches)
     float4 *pos = nullptr;
 
     // per-tick buffers
@@ -231,6 +232,7 @@ struct gr_fa2 {
             cudaStreamDestroy(stream);
         }
     }
+    Segments segments() const { return Segments{nseg, seg_row, seg_first, seg_out, seg_done}; }
     // k_bounds runs k_update's grid, so that the update can compute the same bounds
     uint32_t bnd_blocks() const { return frc_blocks(n); }
 };
@@ -778,8 +780,10 @@ static int build_segments(gr_fa2 *h) {
     CU(cudaStreamSynchronize(s));
     h->nseg = nseg;
     if (!nseg) return GR_OK;
-    if ((e = h->alloc(&h->seg_row, nseg)) || (e = h->alloc(&h->seg_out, (size_t)nseg * h->dim)))
+    if ((e = h->alloc(&h->seg_row, nseg)) || (e = h->alloc(&h->seg_out, (size_t)nseg * h->dim)) ||
+        (e = h->alloc(&h->seg_done, nseg)))
         return set_err(GR_ALLOC_FAILED, cudaGetErrorString(e));
+    cudaMemsetAsync(h->seg_done, 0, (size_t)nseg * 4, s);
     k_seg_fill<<<div_up(n, 256), 256, 0, s>>>(n, h->rp, LIGHT_MAX, SEG, h->seg_first, h->seg_row);
     CU(cudaGetLastError());
     return GR_OK;
@@ -1554,7 +1558,7 @@ static int forces_static(uint32_t n, const float4 *nodes, const uint32_t *rp, co
     h.wt = const_cast<float *>(wt);
     h.pos = const_cast<float4 *>(nodes);
     h.U = out;
-    // seg_first stays null: every row takes the row loop.
+    // nseg stays 0: every row takes the row sums
     k_static_init<<<1, 1, 0, s>>>(h.st, tick);
     enqueue_tick<D>(&h, true, PH_ALL);
     cudaError_t e = cudaGetLastError();
@@ -2442,7 +2446,7 @@ struct gr_force_session {
     double *box_part = nullptr;
     int table_level = 0;
     double widest = 0.0;          // more than any pair in reach is apart on one axis
-    float2 *vel = nullptr, *seg_out = nullptr;
+    float2 *vel = nullptr;
     D3State *ds = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -2528,12 +2532,8 @@ void d3_enqueue(gr_force_session *S) {
     gr_fa2 *t = S->t;
     cudaStream_t s = t->stream;
     const uint32_t n = S->n, g = div_up(n, D3_T);
-    k_d3_project<<<g, D3_T, 0, s>>>(n, S->p4, S->vel, t->rp, S->pp4, S->ds, S->prm.alpha_decay);
-    if (t->nseg)
-        k_d3_link_seg<<<div_up((uint64_t)t->nseg * GR_WARP, D3_T), D3_T, 0, s>>>(
-            S->P, t->nseg, S->ds, S->pp4, t->rp, S->lk, t->seg_row, t->seg_first, S->seg_out);
-    k_d3_link<<<g, D3_T, 0, s>>>(S->P, S->ds, S->pp4, t->rp, S->lk, t->nseg ? t->seg_first : nullptr, S->seg_out,
-                                 S->vel);
+    k_d3_project<<<g, D3_T, 0, s>>>(n, S->p4, S->vel, S->pp4, S->ds, S->prm.alpha_decay);
+    k_d3_link<<<rows_grid(n, t->nseg), FRC_THREADS, 0, s>>>(S->P, S->ds, S->pp4, t->rp, S->lk, t->segments(), S->vel);
     const double *mean;
     if (S->mesh) {  // many-body on the particle mesh
         pm_enqueue(S);
@@ -2541,7 +2541,7 @@ void d3_enqueue(gr_force_session *S) {
     } else {  // many-body: the tree of the positions
         t->pos = S->p4;
         enqueue_tick<2>(t, false, PH_TREE);
-        k_d3_charge<<<g, D3_T, 0, s>>>(S->P, S->ds, t->st, t->cells, t->sp, t->sorig, S->vel);
+        (t->cells.skip ? k_d3_charge<true> : k_d3_charge<false>)<<<g, D3_T, 0, s>>>(S->P, S->ds, t->st, t->cells, t->sp, t->sorig, S->vel);
         mean = t->st->mean;
     }
     ZeroWords zw;
@@ -2655,7 +2655,7 @@ int gr_force_session_create(gr_force_session **out, uint32_t n, uint64_t m, cons
     }
     if ((e = t->alloc(&S->p4, n)) || (e = t->alloc(&S->pp4, n)) || (e = t->alloc(&S->lk, ne)) ||
         (e = t->alloc(&S->grid, 1)) || (e = t->alloc(&S->box_part, 4 * (size_t)D3_CENTER_BLOCKS)) ||
-        (e = t->alloc(&S->table, (size_t)1 << (2 * S->table_level))) || (e = t->alloc(&S->vel, n)) || (e = t->alloc(&S->seg_out, std::max<uint32_t>(t->nseg, 1))) ||
+        (e = t->alloc(&S->table, (size_t)1 << (2 * S->table_level))) || (e = t->alloc(&S->vel, n)) ||
         (e = t->alloc(&S->ds, 1))) {
         delete S;
         return set_err(GR_ALLOC_FAILED, cudaGetErrorString(e));

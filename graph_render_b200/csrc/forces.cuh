@@ -210,6 +210,157 @@ k_attract(uint32_t n, int lin_log, const DevState *st, const float4 *__restrict_
     if (D == 3) att[(size_t)i * D + 2] = a2;
 }
 
+// ---- sums over CSR rows whose terms cost a square root and a quotient. A warp
+// takes 32 consecutive rows: its lanes compute the terms of all their entries side
+// by side (consecutive entries, whatever the rows' lengths), ROWS_WIN at a time
+// into shared memory, and each lane then adds its own row's in entry order, the
+// sum a loop over the row gives. One lane a row, the lanes wait for the longest of
+// 32 rows, each entry's loads and arithmetic in one serial chain: d3-force's link
+// pass at 1M nodes and 3.1M entries took 79 us that way and 43 this way. FA2's
+// attraction stays a lane a row: its linear term costs little beside its gather
+// (unit weights over 8M entries: 56 us, spread 69), and the row sums run beside
+// the walk, whose pipe the shared memory's traffic shares (a 1M-node tick 40 us
+// longer).
+constexpr int ROWS_WIN = 128;
+
+template <int D>
+struct RowsShared {  // one warp's
+    float4 p[GR_WARP];
+    uint32_t pre[GR_WARP], base[GR_WARP];
+    float v[D + 1][ROWS_WIN];
+};
+
+// acc += the terms of this lane's row (row0 + lane): `len` entries from e0, p its
+// record. term(p, row, e, q, d) gives the factor of entry e, whose neighbour's
+// record is q, and its D components in d. The whole warp calls it.
+template <int D, typename Col, typename Term>
+__device__ __forceinline__ void warp_rows(RowsShared<D> &S, uint32_t row0, const float4 &p, uint32_t e0,
+                                          uint32_t len, float *acc, const float4 *__restrict__ pos, Col col, Term term) {
+    const uint32_t lane = threadIdx.x % GR_WARP;
+    uint32_t inc = len;
+#pragma unroll
+    for (int o = 1; o < GR_WARP; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(GR_FULL, inc, o);
+        if (lane >= (uint32_t)o) inc += y;
+    }
+    const uint32_t total = __shfl_sync(GR_FULL, inc, GR_WARP - 1), pre = inc - len;
+    S.p[lane] = p;
+    S.pre[lane] = pre;
+    S.base[lane] = e0 - pre;
+    __syncwarp();
+    for (uint32_t w0 = 0; w0 < total; w0 += ROWS_WIN) {
+#pragma unroll
+        for (int u = 0; u < ROWS_WIN / GR_WARP; u++) {
+            const uint32_t slot = u * GR_WARP + lane, t = w0 + slot;
+            if (t < total) {
+                uint32_t r = 0;  // the last row that begins at or before t
+#pragma unroll
+                for (uint32_t h = GR_WARP / 2; h >= 1; h >>= 1)
+                    if (S.pre[r + h] <= t) r += h;
+                float d[D];
+                const uint32_t e = t + S.base[r];
+                const float c = term(S.p[r], row0 + r, e, pos[col(e)], d);
+#pragma unroll
+                for (int a = 0; a < D; a++) S.v[a][slot] = d[a];
+                S.v[D][slot] = c;
+            }
+        }
+        __syncwarp();
+        const uint32_t t1 = min(pre + len, w0 + ROWS_WIN);
+        for (uint32_t t = max(pre, w0); t < t1; t++) {
+            const float c = S.v[D][t - w0];
+#pragma unroll
+            for (int a = 0; a < D; a++) acc[a] = __fmaf_rn(S.v[a][t - w0], c, acc[a]);
+        }
+        __syncwarp();
+    }
+}
+
+// Rows of more than LIGHT_MAX entries are summed in SEG-entry segments, one warp
+// each (lanes stride by 32, then a fixed butterfly); the warp that finishes a
+// row's last segment adds the segment sums in segment order. `done` counts a row's
+// finished segments at the index of its first one, and is 0 again afterwards.
+// Returns whether this lane holds the row's sum in acc (lane 0 of that warp).
+template <int D, typename Col, typename Term>
+__device__ __forceinline__ bool warp_segment(uint32_t s, uint32_t row, uint32_t first, uint32_t r0, uint32_t r1,
+                                             float *seg_out, uint32_t *done, float *acc,
+                                             const float4 *__restrict__ pos, Col col, Term term) {
+    const uint32_t lane = threadIdx.x % GR_WARP;
+    const uint32_t e0 = r0 + (s - first) * SEG, e1 = min(e0 + SEG, r1);
+#pragma unroll
+    for (int a = 0; a < D; a++) acc[a] = 0.f;
+    const float4 p = pos[row];
+    for (uint32_t e = e0 + lane; e < e1; e += GR_WARP) {
+        float d[D];
+        const float c = term(p, row, e, pos[col(e)], d);
+#pragma unroll
+        for (int a = 0; a < D; a++) acc[a] = __fmaf_rn(d[a], c, acc[a]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int a = 0; a < D; a++) acc[a] += __shfl_xor_sync(GR_FULL, acc[a], o);
+    if (lane != 0) return false;
+#pragma unroll
+    for (int a = 0; a < D; a++) __stcg(&seg_out[(size_t)s * D + a], acc[a]);
+    __threadfence();
+    const uint32_t ns = (r1 - r0 + SEG - 1) / SEG;
+    if (atomicAdd(&done[first], 1u) != ns - 1) return false;
+    __threadfence();
+    done[first] = 0u;
+#pragma unroll
+    for (int a = 0; a < D; a++) acc[a] = 0.f;
+    for (uint32_t k = first; k < first + ns; k++)
+#pragma unroll
+        for (int a = 0; a < D; a++) acc[a] += __ldcg(&seg_out[(size_t)k * D + a]);
+    return true;
+}
+
+// A graph's heavy rows, none when count is 0.
+struct Segments {
+    uint32_t count;
+    const uint32_t *row, *first;  // segment -> row, row -> its first segment
+    float *out;                   // D a segment
+    uint32_t *done;               // zero
+};
+
+__host__ __device__ inline uint32_t seg_blocks(uint32_t count) {
+    return (uint32_t)(((uint64_t)count * GR_WARP + FRC_THREADS - 1) / FRC_THREADS);
+}
+__host__ __device__ inline uint32_t rows_grid(uint32_t n, uint32_t segs) {
+    return seg_blocks(segs) + (n + FRC_THREADS - 1) / FRC_THREADS;
+}
+
+// Every row's sum of term over its CSR entries, by blocks of FRC_THREADS threads:
+// the segments' blocks first, then one lane a row with the warp's lanes
+// sharing the terms. col(e) is entry e's neighbour; put(row, acc) takes each sum.
+template <int D, typename Col, typename Term, typename Put>
+__device__ __forceinline__ void block_rows(uint32_t n, const float4 *__restrict__ pos, const uint32_t *__restrict__ rp,
+                                           const Segments &G, Col col, Term term, Put put) {
+    const uint32_t sb = seg_blocks(G.count);
+    float acc[D];
+    if (blockIdx.x < sb) {
+        const uint32_t s = (blockIdx.x * FRC_THREADS + threadIdx.x) / GR_WARP;
+        if (s >= G.count) return;
+        const uint32_t row = G.row[s];
+        if (warp_segment<D>(s, row, G.first[row], rp[row], rp[row + 1], G.out, G.done, acc, pos, col, term)) put(row, acc);
+        return;
+    }
+    const uint32_t i = (blockIdx.x - sb) * FRC_THREADS + threadIdx.x, row0 = i & ~(GR_WARP - 1u);
+    if (row0 >= n) return;
+    const bool valid = i < n;
+    const uint32_t e0 = valid ? rp[i] : 0u;
+    uint32_t len = valid ? rp[i + 1] - e0 : 0u;
+    const bool heavy = G.count != 0u && len > LIGHT_MAX;
+    if (heavy) len = 0u;
+    const float4 p = valid ? pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int a = 0; a < D; a++) acc[a] = 0.f;
+    __shared__ RowsShared<D> s_rows[FRC_THREADS / GR_WARP];
+    warp_rows<D>(s_rows[threadIdx.x / GR_WARP], row0, p, e0, len, acc, pos, col, term);
+    if (valid && !heavy) put(i, acc);
+}
+
 // u_i for every node from its attraction (read from U, where k_attract put it;
 // each thread reads and then overwrites only its own node's entries) and its
 // repulsion; per-block FP64 swing and traction; the last block accumulates
