@@ -2457,8 +2457,9 @@ struct gr_force_session {
     PmState *pm = nullptr;
     double *pm_part = nullptr;
     uint64_t *pm_key = nullptr;
-    uint32_t *pm_val = nullptr, *pm_cs = nullptr, *pm_ce = nullptr;
-    float2 *pm_frac = nullptr, *ga = nullptr, *gk = nullptr, *gt = nullptr, *tw = nullptr;
+    uint32_t *pm_val = nullptr;
+    uint2 *pm_table = nullptr;
+    float2 *pm_frac = nullptr, *pm_sfrac = nullptr, *ga = nullptr, *gk = nullptr, *gt = nullptr, *tw = nullptr;
     RadixSorter pm_sorter;
     ~gr_force_session() {
         pm_sorter.release();
@@ -2488,43 +2489,52 @@ int d3_validate(const gr_force_params &p) {
 }
 
 // The mesh's many-body pass (pm.cuh): frame, stencils, cell sort, deposit,
-// Green's function, forward FFTs (spectra transposed), product, inverse FFT
-// (natural layout), bilinear read onto the velocities.
-void pm_fft2(gr_force_session *S, float2 *a, float2 *scratch, bool inverse, cudaStream_t s) {
-    const uint32_t side = S->side, th = std::min<uint32_t>(side / 2, 512);
-    const size_t sm = (size_t)side * sizeof(float2);
-    const dim3 tg(side / 32, side / 32), tb(32, 8);
-    if (inverse) {
-        k_pm_fft_rows<true><<<side, th, sm, s>>>(a, S->tw, side, S->bits, S->pm);
-        k_pm_transpose<<<tg, tb, 0, s>>>(a, scratch, side, S->pm);
-        k_pm_fft_rows<true><<<side, th, sm, s>>>(scratch, S->tw, side, S->bits, S->pm);
-    } else {
-        k_pm_fft_rows<false><<<side, th, sm, s>>>(a, S->tw, side, S->bits, S->pm);
-        k_pm_transpose<<<tg, tb, 0, s>>>(a, scratch, side, S->pm);
-        k_pm_fft_rows<false><<<side, th, sm, s>>>(scratch, S->tw, side, S->bits, S->pm);
-    }
+// convolution, bilinear read onto the velocities.
+
+// The convolution of the deposited density (ga) with the law's Green's function,
+// into ga.
+template <int BITS>
+void pm_convolve(gr_force_session *S, double dmin2, double dmax2, cudaStream_t s) {
+    using F = Fft<BITS>;
+    auto launch = [&](auto k, uint32_t blocks, auto... args) {
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F::SMEM);
+        k<<<blocks, F::THREADS, F::SMEM, s>>>(args...);
+    };
+    const uint32_t blocks = F::N / FFT_ROWS;
+    launch(k_pm_fft_forward<BITS>, 2 * blocks, (const float2 *)S->ga, S->gk, S->gt, (const float2 *)S->tw,
+           (const PmState *)S->pm, dmin2, dmax2);
+    launch(k_pm_fft_middle<BITS>, blocks, (const float2 *)S->gk, (const float2 *)S->gt, S->ga, (const float2 *)S->tw,
+           (const PmState *)S->pm);
+    launch(k_pm_fft_inverse<BITS>, blocks, S->ga, (const float2 *)S->tw, (const PmState *)S->pm);
 }
 
 void pm_enqueue(gr_force_session *S) {
     cudaStream_t s = S->t->stream;
     const uint32_t n = S->n, side = S->side, g = div_up(n, PM_T);
-    const uint32_t mg = div_up(side * side, PM_T);
     const double dmin2 = S->prm.distance_min * S->prm.distance_min;
     const double dmax2 = S->prm.distance_max * S->prm.distance_max;
-    k_pm_bounds<<<S->pm_blocks, PM_T, 0, s>>>(n, S->p4, side, S->prm.distance_max, dmax2, S->pm_part, S->pm);
-    k_pm_stencil<<<g, PM_T, 0, s>>>(n, S->p4, S->pm, side, S->pm_key, S->pm_val, S->pm_frac);
-    // cell keys are row-major indices below side^2: 2 x bits significant bits, one-sweep
-    // passes (a wait that gives up is reported through the tree handle's state)
-    S->pm_sorter.sort_bits(S->pm_key, S->pm_val, n, 2 * (int)S->bits, s, &S->t->st->error);
-    cudaMemsetAsync(S->pm_cs, 0, (size_t)side * side * 4, s);
-    cudaMemsetAsync(S->pm_ce, 0, (size_t)side * side * 4, s);
-    k_pm_mark<<<g, PM_T, 0, s>>>(n, S->pm, S->pm_key, S->pm_cs, S->pm_ce);
-    k_pm_deposit<<<mg, PM_T, 0, s>>>(side, S->pm, S->pm_cs, S->pm_ce, S->pm_val, S->pm_frac, S->ga);
-    k_pm_green<<<mg, PM_T, 0, s>>>(side, S->pm, dmin2, dmax2, S->gk);
-    pm_fft2(S, S->gk, S->gt, false, s);  // kernel spectrum, transposed, in gt
-    pm_fft2(S, S->ga, S->gk, false, s);  // density spectrum, transposed, in gk
-    k_pm_mul<<<mg, PM_T, 0, s>>>(side * side, S->gk, S->gt, S->pm);
-    pm_fft2(S, S->gk, S->ga, true, s);   // field, natural layout, in ga
+    RadixSorter &o = S->pm_sorter;
+    ZeroWords zw;
+    zw.add(o.os_ghist, RadixSorter::ghist_words());
+    k_pm_bounds<<<S->pm_blocks, PM_T, 0, s>>>(n, S->p4, side, S->prm.distance_max, dmax2, S->pm_part, S->pm, zw,
+                                              S->pm_table);
+    // cell keys are row-major indices below side^2, 14 to 20 bits: two or three
+    // one-sweep passes (a wait that gives up is reported through the tree handle's
+    // state). The sorter's scratch pair holds the input of an odd count.
+    const int passes = 2 * (int)S->bits > 16 ? 3 : 2;
+    const uint64_t words = (uint64_t)passes * div_up(n, os_tile_keys(n)) * RS_BINS;
+    uint64_t *k0 = passes & 1 ? o.k_alt : S->pm_key;
+    uint32_t *v0 = passes & 1 ? o.v_alt : S->pm_val;
+    (passes == 3 ? k_pm_stencil<3> : k_pm_stencil<2>)<<<std::min<uint32_t>(div_up(n, PM_T * 2), 4 * 148), PM_T, 0, s>>>(
+        n, S->p4, S->pm, side, k0, v0, S->pm_frac, o.os_ghist, o.os_status, words);
+    o.onesweep_passes(S->pm_key, S->pm_val, n, 0, passes, s, &S->t->st->error, &S->pm->skip, S->t->pdl,
+                      &S->t->st->converged);
+    k_pm_mark<<<g, PM_T, 0, s>>>(n, S->pm, S->pm_key, S->pm_val, S->pm_frac, S->pm_table, S->pm_sfrac);
+    k_pm_deposit<<<div_up(side * side, PM_T), PM_T, 0, s>>>(side, S->pm, S->pm_table, S->pm_sfrac, S->ga);
+    if (S->bits == 10) pm_convolve<10>(S, dmin2, dmax2, s);
+    else if (S->bits == 9) pm_convolve<9>(S, dmin2, dmax2, s);
+    else if (S->bits == 8) pm_convolve<8>(S, dmin2, dmax2, s);
+    else pm_convolve<7>(S, dmin2, dmax2, s);
     k_pm_read<<<g, PM_T, 0, s>>>(n, S->p4, S->pm, side, (float)S->prm.charge, &S->ds->alpha, S->ga, S->vel);
 }
 
@@ -2812,7 +2822,7 @@ int gr_force_session_use_mesh(gr_force_session *S) {
     cudaError_t e;
     if ((e = t->alloc(&S->pm, 1)) || (e = t->alloc(&S->pm_part, 6 * (size_t)blocks)) ||
         (e = t->alloc(&S->pm_key, n)) || (e = t->alloc(&S->pm_val, n)) || (e = t->alloc(&S->pm_frac, n)) ||
-        (e = t->alloc(&S->pm_cs, NN)) || (e = t->alloc(&S->pm_ce, NN)) || (e = t->alloc(&S->ga, NN)) ||
+        (e = t->alloc(&S->pm_table, NN)) || (e = t->alloc(&S->pm_sfrac, n)) || (e = t->alloc(&S->ga, NN)) ||
         (e = t->alloc(&S->gk, NN)) || (e = t->alloc(&S->gt, NN)) || (e = t->alloc(&S->tw, side / 2)) ||
         (e = S->pm_sorter.init(std::max<uint32_t>(n, 1), t->stream, true)))
         return set_err(GR_ALLOC_FAILED, cudaGetErrorString(e));

@@ -9,12 +9,13 @@
 // FP64 in the last block of the bounds pass. The deposit is a gather: nodes are
 // radix-sorted by their cell, and every mesh point sums the nodes of the four
 // cells that touch it in a fixed order, so the density is the same every run.
-// The FFT is radix-2 in shared memory along rows, with a tiled transpose between
-// the two directions; spectra stay transposed, so the inverse's transpose
-// restores the natural layout. FP32 mesh values, FP64 frame.
+// The FFT's radix-2 stages run along rows, three at a time in registers; each
+// direction's pass writes its rows as columns, so spectra stay transposed and the
+// inverse's first pass restores the natural layout. FP32 mesh values, FP64 frame.
 #pragma once
 
 #include "common.cuh"
+#include "tree.cuh"
 
 namespace gr {
 
@@ -28,13 +29,17 @@ struct PmState {
     int32_t step;
     uint32_t cells, reach, valid;
     uint32_t ticket;
+    uint32_t skip;  // 1 when the frame is not valid: the sort's passes do nothing
 };
 
 // Extent (finite points) and FP64 coordinate sums; the last block folds the
-// block partials in block order, places the frame and takes the mean.
+// block partials in block order, places the frame and takes the mean. Also zeroes
+// the cell sort's counters and the cell table.
 __global__ void __launch_bounds__(PM_T)
 k_pm_bounds(uint32_t n, const float4 *__restrict__ p, uint32_t side, double dmax, double dmax2,
-            double *__restrict__ part, PmState *S) {
+            double *__restrict__ part, PmState *S, ZeroWords zw, uint2 *__restrict__ table) {
+    if (blockIdx.x == 0) zw.clear();
+    for (uint32_t i = blockIdx.x * PM_T + threadIdx.x; i < side * side; i += gridDim.x * PM_T) table[i] = make_uint2(0u, 0u);
     __shared__ double s_red[PM_T / GR_WARP];
     __shared__ bool s_last;
     double lx = INFINITY, ly = INFINITY, hx = -INFINITY, hy = -INFINITY, sx = 0.0, sy = 0.0;
@@ -123,6 +128,7 @@ k_pm_bounds(uint32_t n, const float4 *__restrict__ p, uint32_t side, double dmax
     S->mean[0] = n ? X / (double)n : 0.0;
     S->mean[1] = n ? Y / (double)n : 0.0;
     S->valid = 0u;
+    S->skip = 1u;
     const double span = fmax(H0 - L0, H1 - L1);
     if (n < 2 || !(dmax2 > 0.0) || !(L0 <= H0) || !isfinite(span)) return;
     int step = (int)floor(4.0 * log2(span / (double)side));
@@ -142,6 +148,7 @@ k_pm_bounds(uint32_t n, const float4 *__restrict__ p, uint32_t side, double dmax
         S->ox = floor(L0 / h) * h;
         S->oy = floor(L1 / h) * h;
         S->valid = 1u;
+        S->skip = 0u;
         return;
     }
 }
@@ -159,50 +166,75 @@ __device__ __forceinline__ void pm_split(const PmState &S, float px, float py, u
     fy = (float)fmin(fmax(u1 - (double)c1, 0.0), 1.0);
 }
 
-// Each node's cell key (row-major) and fractions, for the sort and the deposit.
-__global__ void k_pm_stencil(uint32_t n, const float4 *__restrict__ p, const PmState *S, uint32_t side,
-                             uint64_t *__restrict__ key, uint32_t *__restrict__ val, float2 *__restrict__ frac) {
-    const uint32_t i = blockIdx.x * PM_T + threadIdx.x;
-    if (i >= n || !S->valid) return;
-    uint32_t cx, cy;
-    float fx, fy;
-    const float4 a = p[i];
-    pm_split(*S, a.x, a.y, cx, cy, fx, fy);
-    key[i] = (uint64_t)cy * side + cx;
-    val[i] = i;
-    frac[i] = make_float2(fx, fy);
+// Each node's cell key (row-major) and fractions, the digit counts of the keys'
+// low PASSES bytes and the zeroing of those passes' look-back words.
+template <int PASSES>
+__global__ void __launch_bounds__(PM_T)
+k_pm_stencil(uint32_t n, const float4 *__restrict__ p, const PmState *S, uint32_t side, uint64_t *__restrict__ key,
+             uint32_t *__restrict__ val, float2 *__restrict__ frac, uint32_t *__restrict__ ghist,
+             uint32_t *__restrict__ status, uint64_t status_words) {
+    static_assert(PM_T == 256, "one thread per digit");
+    if (!S->valid) return;
+    __shared__ uint32_t s_h[PASSES][256];
+    const int t = threadIdx.x;
+#pragma unroll
+    for (int q = 0; q < PASSES; q++) s_h[q][t] = 0;
+    __syncthreads();
+    const uint64_t stride = (uint64_t)gridDim.x * PM_T, first = (uint64_t)blockIdx.x * PM_T + t;
+    for (uint64_t i = first; i < n; i += stride) {
+        uint32_t cx, cy;
+        float fx, fy;
+        const float4 a = p[i];
+        pm_split(*S, a.x, a.y, cx, cy, fx, fy);
+        const uint32_t k = cy * side + cx;
+        key[i] = k;
+        val[i] = (uint32_t)i;
+        frac[i] = make_float2(fx, fy);
+#pragma unroll
+        for (int q = 0; q < PASSES; q++) atomicAdd(&s_h[q][(k >> (8 * q)) & 0xffu], 1u);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < PASSES; q++)
+        if (s_h[q][t]) atomicAdd(&ghist[q * 256 + t], s_h[q][t]);
+    for (uint64_t i = first; i < status_words; i += stride) status[i] = 0u;
 }
 
 // First and one-past-last sorted position of every occupied cell (the others
-// were cleared to 0, 0).
-__global__ void k_pm_mark(uint32_t n, const PmState *S, const uint64_t *__restrict__ key, uint32_t *__restrict__ cs,
-                          uint32_t *__restrict__ ce) {
+// were cleared to 0, 0), and the fractions in sorted order.
+__global__ void k_pm_mark(uint32_t n, const PmState *S, const uint64_t *__restrict__ key,
+                          const uint32_t *__restrict__ val, const float2 *__restrict__ frac, uint2 *__restrict__ table,
+                          float2 *__restrict__ sfrac) {
     const uint32_t q = blockIdx.x * PM_T + threadIdx.x;
     if (q >= n || !S->valid) return;
     const uint64_t k = key[q];
-    if (q == 0 || key[q - 1] != k) cs[k] = q;
-    if (q + 1 == n || key[q + 1] != k) ce[k] = q + 1;
+    sfrac[q] = frac[val[q]];
+    if (q == 0 || key[q - 1] != k) table[k].x = q;
+    if (q + 1 == n || key[q + 1] != k) table[k].y = q + 1;
 }
 
 // deposit.rs: mesh point (gx, gy) gathers the cloud-in-cell weights of the nodes
 // in the four cells touching it, cell by cell in a fixed order, nodes in sorted
 // order. Writes the whole mesh (zero where nothing lands).
-__global__ void k_pm_deposit(uint32_t side, const PmState *S, const uint32_t *__restrict__ cs,
-                             const uint32_t *__restrict__ ce, const uint32_t *__restrict__ val,
-                             const float2 *__restrict__ frac, float2 *__restrict__ mesh) {
+__global__ void k_pm_deposit(uint32_t side, const PmState *S, const uint2 *__restrict__ table,
+                             const float2 *__restrict__ sfrac, float2 *__restrict__ mesh) {
     const uint32_t g = blockIdx.x * PM_T + threadIdx.x;
     if (g >= side * side) return;
     float acc = 0.f;
     if (S->valid) {
         const int gx = (int)(g % side), gy = (int)(g / side), top = (int)S->cells - 2;
+        uint2 r[4];
 #pragma unroll
         for (int c = 0; c < 4; c++) {
             const int sx = gx - 1 + (c & 1), sy = gy - 1 + (c >> 1);  // source cell
-            if (sx < 0 || sy < 0 || sx > top || sy > top) continue;
+            const bool in = sx >= 0 && sy >= 0 && sx <= top && sy <= top;
+            r[c] = in ? __ldg(&table[(uint32_t)sy * side + (uint32_t)sx]) : make_uint2(0u, 0u);
+        }
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
             const bool xplus = (c & 1) == 0, yplus = (c >> 1) == 0;  // g is the source's +1 corner on that axis
-            const uint32_t cell = (uint32_t)sy * side + (uint32_t)sx;
-            for (uint32_t q = cs[cell]; q < ce[cell]; q++) {
-                const float2 f = frac[val[q]];
+            for (uint32_t q = r[c].x; q < r[c].y; q++) {
+                const float2 f = __ldg(&sfrac[q]);
                 acc += (xplus ? f.x : 1.f - f.x) * (yplus ? f.y : 1.f - f.y);
             }
         }
@@ -210,72 +242,194 @@ __global__ void k_pm_deposit(uint32_t side, const PmState *S, const uint32_t *__
     mesh[g] = make_float2(acc, 0.f);
 }
 
-// kernel.rs sample + green: the law's vector Green's function at every mesh
-// offset within reach (wrapped), scaled by 1 / side^2; zero elsewhere.
-__global__ void k_pm_green(uint32_t side, const PmState *S, double dmin2, double dmax2, float2 *__restrict__ g) {
-    const uint32_t q = blockIdx.x * PM_T + threadIdx.x;
-    if (q >= side * side) return;
-    float2 out = make_float2(0.f, 0.f);
-    if (S->valid) {
-        const int reach = (int)S->reach, c = (int)(q % side), r = (int)(q / side), sd = (int)side;
-        // a wrapped index both offsets reach is written by the positive one (the later write)
-        const int dx = c <= reach ? c : (c >= sd - reach ? c - sd : INT32_MIN);
-        const int dy = r <= reach ? r : (r >= sd - reach ? r - sd : INT32_MIN);
-        if (dx != INT32_MIN && dy != INT32_MIN) {
-            const double rx = (double)dx * S->h, ry = (double)dy * S->h;
-            double l = rx * rx + ry * ry;
-            if (l != 0.0 && l < dmax2) {
-                if (l < dmin2) l = sqrt(dmin2 * l);
-                const double scale = 1.0 / ((double)side * (double)side);
-                out = make_float2((float)(-rx / l * scale), (float)(-ry / l * scale));
-            }
-        }
-    }
-    g[q] = out;
+// kernel.rs sample + green: the law's vector Green's function at mesh offset
+// (c, r) within reach (wrapped), scaled by 1 / side^2; zero elsewhere.
+__device__ __forceinline__ float2 pm_green(const PmState &S, int side, int c, int r, double dmin2, double dmax2) {
+    const int reach = (int)S.reach;
+    // a wrapped index both offsets reach is written by the positive one (the later write)
+    const int dx = c <= reach ? c : (c >= side - reach ? c - side : INT32_MIN);
+    const int dy = r <= reach ? r : (r >= side - reach ? r - side : INT32_MIN);
+    if (dx == INT32_MIN || dy == INT32_MIN) return make_float2(0.f, 0.f);
+    const double rx = (double)dx * S.h, ry = (double)dy * S.h;
+    double l = rx * rx + ry * ry;
+    if (!(l != 0.0 && l < dmax2)) return make_float2(0.f, 0.f);
+    if (l < dmin2) l = sqrt(dmin2 * l);
+    const double scale = 1.0 / ((double)side * (double)side);
+    return make_float2((float)(-rx / l * scale), (float)(-ry / l * scale));
 }
 
-// One radix-2 transform per row (one block per row), in shared memory:
-// bit-reversed load, log2(side) butterfly stages, twiddles tw[k] = e^(-2 pi i k
-// / side) (conjugated for the inverse); neither direction is scaled.
-template <bool INV>
-__global__ void k_pm_fft_rows(float2 *__restrict__ data, const float2 *__restrict__ tw, uint32_t side, uint32_t bits,
-                              const PmState *S) {
-    if (!S->valid) return;
-    extern __shared__ float2 pm_row[];
-    float2 *row = data + (size_t)blockIdx.x * side;
-    for (uint32_t i = threadIdx.x; i < side; i += blockDim.x) pm_row[__brev(i) >> (32 - bits)] = row[i];
-    __syncthreads();
-    for (uint32_t m = 1; m < side; m <<= 1) {
-        for (uint32_t b = threadIdx.x; b < side / 2; b += blockDim.x) {
-            const uint32_t k = b % m, i0 = (b / m) * 2 * m + k, i1 = i0 + m;
-            float2 w = tw[k * (side / (2 * m))];
+// ---- the FFT. Radix-2, decimation in time: bit-reversed load, log2(side) stages,
+// twiddles tw[k] = e^(-2 pi i k / side) (conjugated for the inverse); neither
+// direction is scaled. side / 8 threads a row hold eight elements each and run
+// three stages between exchanges through shared memory (a stage's butterflies are
+// the same whichever way its elements are held). A block takes FFT_ROWS rows and
+// writes them as columns, 32 consecutive bytes each, so a direction is one kernel:
+//   k_pm_fft_forward   density rows, and the Green's function's made on the way in
+//   k_pm_fft_middle    their columns, the product, and the inverse's first rows
+//   k_pm_fft_inverse   the inverse's other rows, in place
+// A stage at a time in shared memory with a transpose kernel between directions,
+// six row passes, three transposes, the sampled kernel and the product were eleven
+// kernels of 184 us at side 1024; these are three of 60 us.
+constexpr int FFT_ROWS = 4;
+
+template <int BITS>
+struct Fft {
+    static constexpr uint32_t N = 1u << BITS, TPR = N / 8;    // row length, threads a row
+    static constexpr uint32_t THREADS = FFT_ROWS * TPR;
+    static constexpr uint32_t ROW = N + N / 8 + 16 / FFT_ROWS;  // a padded row: exchanges and columns without bank conflicts
+    static constexpr size_t SMEM = (size_t)(FFT_ROWS * ROW + N / 2) * sizeof(float2);
+};
+
+__device__ __forceinline__ uint32_t fft_pad(uint32_t i) { return i + (i >> 3); }
+
+// c w, each part one product and one fused multiply-add; FIRST: which product of
+// the imaginary part is the fused one (the forward and the inverse transform
+// round it either way, and a tick's chaos shows it within a few ticks).
+template <bool FIRST>
+__device__ __forceinline__ float2 fft_mul(const float2 &c, const float2 &w) {
+    return make_float2(__fmaf_rn(c.x, w.x, -__fmul_rn(c.y, w.y)),
+                       FIRST ? __fmaf_rn(c.x, w.y, __fmul_rn(c.y, w.x)) : __fmaf_rn(c.y, w.x, __fmul_rn(c.x, w.y)));
+}
+
+// Element j of thread t while the index bits S0 .. S0 + 2 are the held ones.
+template <int S0>
+__device__ __forceinline__ uint32_t fft_index(uint32_t t, uint32_t j) {
+    return (t >> S0 << (S0 + 3)) | (j << S0) | (t & ((1u << S0) - 1u));
+}
+
+// Stages CUR .. BITS - 1 of one row; x holds the elements of fft_index<S0> with
+// S0 = min(CUR, BITS - 3), at the end those of fft_index<BITS - 3> (t + j TPR).
+template <int BITS, bool INV, int CUR>
+__device__ __forceinline__ void fft_stages(float2 *x, float2 *row, const float2 *tw, uint32_t t) {
+    constexpr int S0 = CUR < BITS - 3 ? CUR : BITS - 3;
+#pragma unroll
+    for (int s = CUR; s < S0 + 3; s++) {
+        const int b = s - S0;
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            if (j & (1 << b)) continue;
+            const uint32_t k = fft_index<S0>(t, j) & ((1u << s) - 1u);
+            float2 w = tw[k << (BITS - 1 - s)];
             if (INV) w.y = -w.y;
-            const float2 a = pm_row[i0], c = pm_row[i1];
-            const float2 t = make_float2(c.x * w.x - c.y * w.y, c.x * w.y + c.y * w.x);
-            pm_row[i0] = make_float2(a.x + t.x, a.y + t.y);
-            pm_row[i1] = make_float2(a.x - t.x, a.y - t.y);
+            const float2 a = x[j], c = x[j | (1 << b)];
+            const float2 u = fft_mul<!INV>(c, w);
+            x[j] = make_float2(a.x + u.x, a.y + u.y);
+            x[j | (1 << b)] = make_float2(a.x - u.x, a.y - u.y);
         }
-        __syncthreads();
     }
-    for (uint32_t i = threadIdx.x; i < side; i += blockDim.x) row[i] = pm_row[i];
+    if constexpr (S0 + 3 < BITS) {
+        constexpr int N0 = S0 + 3 < BITS - 3 ? S0 + 3 : BITS - 3;
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < 8; j++) row[fft_pad(fft_index<S0>(t, j))] = x[j];
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < 8; j++) x[j] = row[fft_pad(fft_index<N0>(t, j))];
+        fft_stages<BITS, INV, S0 + 3>(x, row, tw, t);
+    }
 }
 
-// out = in^T, 32 x 32 tiles through shared memory.
-__global__ void k_pm_transpose(const float2 *__restrict__ in, float2 *__restrict__ out, uint32_t side,
-                               const PmState *S) {
-    if (!S->valid) return;
-    __shared__ float2 tile[32][33];
-    const uint32_t bx = blockIdx.x * 32, by = blockIdx.y * 32;
-    for (uint32_t j = threadIdx.y; j < 32; j += blockDim.y) tile[j][threadIdx.x] = in[(size_t)(by + j) * side + bx + threadIdx.x];
+// One row's transform: x holds elements t + j TPR before and after. All threads
+// of the block call it together.
+template <int BITS, bool INV>
+__device__ __forceinline__ void fft_row(float2 *x, float2 *row, const float2 *tw, uint32_t t) {
     __syncthreads();
-    for (uint32_t j = threadIdx.y; j < 32; j += blockDim.y) out[(size_t)(bx + j) * side + by + threadIdx.x] = tile[threadIdx.x][j];
+#pragma unroll
+    for (int j = 0; j < 8; j++) row[fft_pad(t + j * Fft<BITS>::TPR)] = x[j];
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 8; j++) x[j] = row[fft_pad(__brev(8 * t + j) >> (32 - BITS))];
+    fft_stages<BITS, INV, 0>(x, row, tw, t);
 }
 
-__global__ void k_pm_mul(uint32_t count, float2 *__restrict__ a, const float2 *__restrict__ b, const PmState *S) {
-    const uint32_t q = blockIdx.x * PM_T + threadIdx.x;
-    if (q >= count || !S->valid) return;
-    const float2 x = a[q], y = b[q];
-    a[q] = make_float2(x.x * y.x - x.y * y.y, x.x * y.y + x.y * y.x);
+// The block's rows r0 .. r0 + FFT_ROWS - 1 as columns of out.
+template <int BITS>
+__device__ __forceinline__ void fft_columns(const float2 *x, float2 *rows, float2 *__restrict__ out, uint32_t r0,
+                                            uint32_t r, uint32_t t) {
+    using F = Fft<BITS>;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 8; j++) rows[r * F::ROW + fft_pad(t + j * F::TPR)] = x[j];
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < F::N * FFT_ROWS; i += F::THREADS)
+        out[(size_t)(i / FFT_ROWS) * F::N + r0 + i % FFT_ROWS] = rows[(i % FFT_ROWS) * F::ROW + fft_pad(i / FFT_ROWS)];
+}
+
+template <int BITS>
+__device__ __forceinline__ float2 *fft_setup(float2 *sm, const float2 *__restrict__ tw) {
+    using F = Fft<BITS>;
+    float2 *s_tw = sm + FFT_ROWS * F::ROW;
+    for (uint32_t i = threadIdx.x; i < F::N / 2; i += F::THREADS) s_tw[i] = tw[i];
+    return s_tw;  // fft_row synchronises before it is read
+}
+
+// Blocks 0 .. N / FFT_ROWS - 1: the density's rows; the others: the Green's
+// function's, which nothing needs in memory before.
+template <int BITS>
+__global__ void __launch_bounds__(Fft<BITS>::THREADS)
+k_pm_fft_forward(const float2 *__restrict__ density, float2 *__restrict__ density_t, float2 *__restrict__ green_t,
+                 const float2 *__restrict__ tw, const PmState *S, double dmin2, double dmax2) {
+    using F = Fft<BITS>;
+    if (!S->valid) return;
+    extern __shared__ float2 pm_sm[];
+    const float2 *s_tw = fft_setup<BITS>(pm_sm, tw);
+    const uint32_t r = threadIdx.x / F::TPR, t = threadIdx.x % F::TPR, blocks = F::N / FFT_ROWS;
+    const bool green = blockIdx.x >= blocks;
+    const uint32_t r0 = (green ? blockIdx.x - blocks : blockIdx.x) * FFT_ROWS;
+    float2 x[8];
+    if (green) {
+#pragma unroll 1
+        for (int j = 0; j < 8; j++)
+            pm_sm[r * F::ROW + fft_pad(t + j * F::TPR)] = pm_green(*S, F::N, (int)(t + j * F::TPR), (int)(r0 + r), dmin2, dmax2);
+#pragma unroll
+        for (int j = 0; j < 8; j++) x[j] = pm_sm[r * F::ROW + fft_pad(t + j * F::TPR)];
+    } else {
+#pragma unroll
+        for (int j = 0; j < 8; j++) x[j] = density[(size_t)(r0 + r) * F::N + t + j * F::TPR];
+    }
+    fft_row<BITS, false>(x, pm_sm + r * F::ROW, s_tw, t);
+    fft_columns<BITS>(x, pm_sm, green ? green_t : density_t, r0, r, t);
+}
+
+template <int BITS>
+__global__ void __launch_bounds__(Fft<BITS>::THREADS)
+k_pm_fft_middle(const float2 *__restrict__ density_t, const float2 *__restrict__ green_t, float2 *__restrict__ field,
+                const float2 *__restrict__ tw, const PmState *S) {
+    using F = Fft<BITS>;
+    if (!S->valid) return;
+    extern __shared__ float2 pm_sm[];
+    const float2 *s_tw = fft_setup<BITS>(pm_sm, tw);
+    const uint32_t r = threadIdx.x / F::TPR, t = threadIdx.x % F::TPR, r0 = blockIdx.x * FFT_ROWS;
+    float2 *row = pm_sm + r * F::ROW;
+    float2 x[8], g[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        g[j] = green_t[(size_t)(r0 + r) * F::N + t + j * F::TPR];
+        x[j] = density_t[(size_t)(r0 + r) * F::N + t + j * F::TPR];
+    }
+    fft_row<BITS, false>(g, row, s_tw, t);
+    fft_row<BITS, false>(x, row, s_tw, t);
+#pragma unroll
+    for (int j = 0; j < 8; j++) x[j] = fft_mul<false>(x[j], g[j]);
+    fft_row<BITS, true>(x, row, s_tw, t);
+    fft_columns<BITS>(x, pm_sm, field, r0, r, t);
+}
+
+template <int BITS>
+__global__ void __launch_bounds__(Fft<BITS>::THREADS)
+k_pm_fft_inverse(float2 *__restrict__ field, const float2 *__restrict__ tw, const PmState *S) {
+    using F = Fft<BITS>;
+    if (!S->valid) return;
+    extern __shared__ float2 pm_sm[];
+    const float2 *s_tw = fft_setup<BITS>(pm_sm, tw);
+    const uint32_t r = threadIdx.x / F::TPR, t = threadIdx.x % F::TPR;
+    float2 *at = field + (size_t)(blockIdx.x * FFT_ROWS + r) * F::N + t;
+    float2 x[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) x[j] = at[j * F::TPR];
+    fft_row<BITS, true>(x, pm_sm + r * F::ROW, s_tw, t);
+#pragma unroll
+    for (int j = 0; j < 8; j++) at[j * F::TPR] = x[j];
 }
 
 // mesh.rs read: the field bilinear at every node, times charge * alpha, onto

@@ -62,6 +62,18 @@ def test_random_cloud_field_matches_the_oracle():
     assert rel(got, o.mesh_field()) < 1e-4
 
 
+@pytest.mark.parametrize("n", [16_384, 16_385, 65_537, 262_145])
+def test_cloud_field_matches_the_oracle_at_every_mesh_side(n):
+    """Sides 128, 256, 512 and 1024: the transform's stages group differently at each. The tolerance is
+    the cloud's above (FP32 transforms of log2(side) stages a direction, 1e-7 each)."""
+    rng = np.random.default_rng(6)
+    p = rng.uniform(0, 45.0 * np.sqrt(n), (n, 2)).astype(np.float32).astype(np.float64)
+    got = gpu_field(p[:, 0], p[:, 1])
+    o = O.D3(n, [], [], [], pos0=p)
+    o.use_mesh()
+    assert rel(got, o.mesh_field()) < 1e-4
+
+
 def test_a_node_out_of_everyones_range_feels_no_force_from_itself():
     f = gpu_field(np.array([0.0, 3000.0]), np.array([0.0, 17.5]))
     assert np.abs(f).max() < 1e-6
