@@ -2229,61 +2229,58 @@ int gr_fa2_adjoint_backward(gr_fa2 *h, const float *dL_dpT, double *dL_dp0, doub
 // ------------------------------------------------------------ stress / BFS --
 //
 // Multi-source BFS and Kruskal stress-1 on the device (stress.cuh). The
-// adjacency of the raw edges (both directions, self-loops dropped) is counted
-// and filled on the host, O(m), and copied once per call.
+// adjacency of the raw edges (both directions, self-loops dropped) is counted,
+// scanned and filled on the device; on the host it was 21 of the 24 ms a stress of
+// 200k nodes and 800k edges took. Edge lists whose entries pass 32-bit offsets are
+// still laid out on the host.
 
 namespace {
 
-struct DevBufs {  // device allocations released on every return path
-    std::vector<void *> p;
+// Device allocations released on every return path: from the stream-ordered pool
+// up to POOL_MAX bytes each, so that what a call leaves in the pool stays bounded.
+struct DevBufs {
+    static constexpr size_t POOL_MAX = 256ull << 20;
+    cudaStream_t s = nullptr;
+    std::vector<void *> pooled, own;
     template <typename T>
     cudaError_t get(T **out, size_t count) {
-        cudaError_t e = cudaMalloc((void **)out, (count ? count : 1) * sizeof(T));
-        if (e == cudaSuccess) p.push_back((void *)*out);
+        const size_t bytes = (count ? count : 1) * sizeof(T);
+        const bool pool = bytes <= POOL_MAX;
+        cudaError_t e = pool ? cudaMallocAsync((void **)out, bytes, s) : cudaMalloc((void **)out, bytes);
+        if (e == cudaSuccess) (pool ? pooled : own).push_back((void *)*out);
         return e;
     }
-    ~DevBufs() {
-        for (void *q : p) cudaFree(q);
+    // opens the stream the buffers belong to
+    cudaError_t open() {
+        keep_pool();
+        return cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
     }
-};
-
-struct StreamGuard {
-    cudaStream_t s = nullptr;
-    ~StreamGuard() {
-        if (s) cudaStreamDestroy(s);
+    ~DevBufs() {
+        for (void *q : pooled) cudaFreeAsync(q, s);
+        if (s) {
+            cudaStreamSynchronize(s);
+            cudaStreamDestroy(s);
+        }
+        for (void *q : own) cudaFree(q);
     }
 };
 
 constexpr uint64_t kMaxHopTableBytes = 16ull << 30;
 
-// Hop counts from the k sources (device) to every node into hops (device, k x n,
-// HOP_NONE when unreachable), 64 sources per level-synchronous pull.
-int bfs_on_device(uint32_t n, uint64_t m, const uint32_t *src, const uint32_t *dst, uint32_t k,
-                  const uint32_t *sources_dev, uint32_t *hops, cudaStream_t s, DevBufs &B) {
-    std::vector<uint64_t> rp((size_t)n + 1, 0);
-    for (uint64_t e = 0; e < m; e++) {
-        if (src[e] >= n || dst[e] >= n) return set_err(GR_INDEX_OUT_OF_RANGE, "edge endpoint out of range", (int)e);
-        if (src[e] == dst[e]) continue;
-        rp[src[e] + 1]++;
-        rp[dst[e] + 1]++;
-    }
-    for (uint32_t i = 0; i < n; i++) rp[i + 1] += rp[i];
-    std::vector<uint32_t> col(std::max<uint64_t>(rp[n], 1));
-    std::vector<uint64_t> fill(rp.begin(), rp.end() - 1);
-    for (uint64_t e = 0; e < m; e++) {
-        if (src[e] == dst[e]) continue;
-        col[fill[src[e]]++] = dst[e];
-        col[fill[dst[e]]++] = src[e];
-    }
-    uint64_t *d_rp;
-    uint32_t *d_col, *d_changed;
+// Hop counts from the k sources over a device adjacency: 64 sources per
+// level-synchronous pull, BFS_AHEAD levels between looks at whether one changed
+// anything (each look is a round trip; a level past the last returns at once).
+constexpr uint32_t BFS_AHEAD = 4;
+
+template <typename Offset>
+int bfs_levels(uint32_t n, const Offset *rp, const uint32_t *col, uint32_t k, const uint32_t *sources_dev,
+               uint32_t *hops, DevBufs &B) {
+    cudaStream_t s = B.s;
+    uint32_t *d_changed;  // [0]: the level before this round; [1 ..]: its own levels
     unsigned long long *vis, *fa, *fb;
     cudaError_t e;
-    if ((e = B.get(&d_rp, (size_t)n + 1)) || (e = B.get(&d_col, col.size())) || (e = B.get(&d_changed, 1)) ||
-        (e = B.get(&vis, n)) || (e = B.get(&fa, n)) || (e = B.get(&fb, n)))
+    if ((e = B.get(&d_changed, BFS_AHEAD + 1)) || (e = B.get(&vis, n)) || (e = B.get(&fa, n)) || (e = B.get(&fb, n)))
         return set_err(GR_ALLOC_FAILED, cudaGetErrorString(e));
-    CU(cudaMemcpyAsync(d_rp, rp.data(), rp.size() * sizeof(uint64_t), cudaMemcpyHostToDevice, s));
-    CU(cudaMemcpyAsync(d_col, col.data(), col.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
     CU(cudaMemsetAsync(hops, 0xff, (size_t)k * n * sizeof(uint32_t), s));
     const uint32_t grid = div_up(n, BFS_T);
     for (uint32_t k0 = 0; k0 < k; k0 += 64) {
@@ -2293,18 +2290,78 @@ int bfs_on_device(uint32_t n, uint64_t m, const uint32_t *src, const uint32_t *d
         CU(cudaMemsetAsync(fa, 0, (size_t)n * 8, s));
         k_msbfs_seed<<<1, 64, 0, s>>>(n, k0, kb, sources_dev, vis, fa, hops);
         unsigned long long *cur = fa, *nxt = fb;
-        for (uint32_t level = 1; level < n; level++) {  // a BFS is at most n - 1 levels deep
+        for (uint64_t level = 1; level < n;) {  // a BFS is at most n - 1 levels deep
+            CU(cudaMemsetAsync(d_changed, 0xff, 4, s));
+            CU(cudaMemsetAsync(d_changed + 1, 0, BFS_AHEAD * 4, s));
+            uint32_t used = 0;
+            for (; used < BFS_AHEAD && level < n; used++, level++) {
+                k_msbfs_level<Offset><<<grid, BFS_T, 0, s>>>(n, rp, col, all, cur, vis, nxt, hops, k0, (uint32_t)level,
+                                                            d_changed + used, d_changed + used + 1);
+                std::swap(cur, nxt);
+            }
             uint32_t changed = 0;
-            CU(cudaMemsetAsync(d_changed, 0, 4, s));
-            k_msbfs_level<<<grid, BFS_T, 0, s>>>(n, d_rp, d_col, all, cur, vis, nxt, hops, k0, level, d_changed);
-            CU(cudaMemcpyAsync(&changed, d_changed, 4, cudaMemcpyDeviceToHost, s));
+            CU(cudaMemcpyAsync(&changed, d_changed + used, 4, cudaMemcpyDeviceToHost, s));
             CU(cudaStreamSynchronize(s));
             if (!changed) break;
-            std::swap(cur, nxt);
         }
     }
     CU(cudaGetLastError());
     return GR_OK;
+}
+
+// Hop counts from the k sources (device) to every node into hops (device, k x n,
+// HOP_NONE when unreachable).
+int bfs_on_device(uint32_t n, uint64_t m, const uint32_t *src, const uint32_t *dst, uint32_t k,
+                  const uint32_t *sources_dev, uint32_t *hops, DevBufs &B) {
+    cudaStream_t s = B.s;
+    cudaError_t e;
+    if (m < (1ull << 30) && n < (1u << 31)) {
+        uint32_t *d_src, *d_dst, *deg, *rp, *col, *bad, first_bad = 0xffffffffu;
+        if ((e = B.get(&d_src, m)) || (e = B.get(&d_dst, m)) || (e = B.get(&deg, (size_t)n + 1)) ||
+            (e = B.get(&rp, (size_t)n + 1)) || (e = B.get(&col, 2 * m)) || (e = B.get(&bad, 1)))
+            return set_err(GR_ALLOC_FAILED, cudaGetErrorString(e));
+        Scanner sc;
+        if ((e = sc.init(n + 1, s, true))) return set_err(GR_ALLOC_FAILED, cudaGetErrorString(e));
+        CU(cudaMemsetAsync(deg, 0, ((size_t)n + 1) * 4, s));
+        CU(cudaMemsetAsync(bad, 0xff, 4, s));
+        if (m) {
+            CU(cudaMemcpyAsync(d_src, src, m * 4, cudaMemcpyHostToDevice, s));
+            CU(cudaMemcpyAsync(d_dst, dst, m * 4, cudaMemcpyHostToDevice, s));
+            k_adj_count<<<div_up(m, BFS_T), BFS_T, 0, s>>>(n, (uint32_t)m, d_src, d_dst, deg, bad);
+        }
+        sc.scan(deg, rp, n + 1, nullptr, 0, nullptr, nullptr, s);
+        sc.release();
+        CU(cudaMemcpyAsync(deg, rp, (size_t)n * 4, cudaMemcpyDeviceToDevice, s));  // the rows' next free entries
+        if (m) k_adj_fill<<<div_up(m, BFS_T), BFS_T, 0, s>>>(n, (uint32_t)m, d_src, d_dst, deg, col);
+        CU(cudaMemcpyAsync(&first_bad, bad, 4, cudaMemcpyDeviceToHost, s));
+        CU(cudaStreamSynchronize(s));
+        if (first_bad != 0xffffffffu)
+            return set_err(GR_INDEX_OUT_OF_RANGE, "edge endpoint out of range", (int)first_bad);
+        return bfs_levels<uint32_t>(n, rp, col, k, sources_dev, hops, B);
+    }
+    std::vector<uint64_t> rp((size_t)n + 1, 0);
+    for (uint64_t q = 0; q < m; q++) {
+        if (src[q] >= n || dst[q] >= n) return set_err(GR_INDEX_OUT_OF_RANGE, "edge endpoint out of range", (int)q);
+        if (src[q] == dst[q]) continue;
+        rp[src[q] + 1]++;
+        rp[dst[q] + 1]++;
+    }
+    for (uint32_t i = 0; i < n; i++) rp[i + 1] += rp[i];
+    std::vector<uint32_t> col(std::max<uint64_t>(rp[n], 1));
+    std::vector<uint64_t> fill(rp.begin(), rp.end() - 1);
+    for (uint64_t q = 0; q < m; q++) {
+        if (src[q] == dst[q]) continue;
+        col[fill[src[q]]++] = dst[q];
+        col[fill[dst[q]]++] = src[q];
+    }
+    uint64_t *d_rp;
+    uint32_t *d_col;
+    if ((e = B.get(&d_rp, (size_t)n + 1)) || (e = B.get(&d_col, col.size())))
+        return set_err(GR_ALLOC_FAILED, cudaGetErrorString(e));
+    CU(cudaMemcpyAsync(d_rp, rp.data(), rp.size() * sizeof(uint64_t), cudaMemcpyHostToDevice, s));
+    CU(cudaMemcpyAsync(d_col, col.data(), col.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+    CU(cudaStreamSynchronize(s));
+    return bfs_levels<uint64_t>(n, d_rp, d_col, k, sources_dev, hops, B);
 }
 
 }  // namespace
@@ -2320,15 +2377,14 @@ int gr_bfs_hops(uint32_t n, uint64_t m, const uint32_t *source, const uint32_t *
         if (sources[i] >= n) return set_err(GR_INDEX_OUT_OF_RANGE, "source out of range", (int)i);
     if (k == 0 || n == 0) return ok();
     DevBufs B;
-    StreamGuard g;
-    CU(cudaStreamCreateWithFlags(&g.s, cudaStreamNonBlocking));
+    CU(B.open());
     uint32_t *d_src, *hops;
     cudaError_t e;
     if ((e = B.get(&d_src, k)) || (e = B.get(&hops, (size_t)k * n))) return set_err(GR_ALLOC_FAILED, cudaGetErrorString(e));
-    CU(cudaMemcpyAsync(d_src, sources, (size_t)k * 4, cudaMemcpyHostToDevice, g.s));
-    if (int c = bfs_on_device(n, m, source, target, k, d_src, hops, g.s, B)) return c;
-    CU(cudaMemcpyAsync(hops_out, hops, (size_t)k * n * 4, cudaMemcpyDeviceToHost, g.s));
-    CU(cudaStreamSynchronize(g.s));
+    CU(cudaMemcpyAsync(d_src, sources, (size_t)k * 4, cudaMemcpyHostToDevice, B.s));
+    if (int c = bfs_on_device(n, m, source, target, k, d_src, hops, B)) return c;
+    CU(cudaMemcpyAsync(hops_out, hops, (size_t)k * n * 4, cudaMemcpyDeviceToHost, B.s));
+    CU(cudaStreamSynchronize(B.s));
     return ok();
 }
 
@@ -2397,8 +2453,7 @@ int gr_stress(uint32_t n, uint64_t m, const uint32_t *source, const uint32_t *ta
     const uint32_t k = (uint32_t)from.size();
     if ((uint64_t)k * n * 4 > kMaxHopTableBytes) return set_err(GR_INVALID_ARGUMENT, "hop table above 16 GiB");
     DevBufs B;
-    StreamGuard g;
-    CU(cudaStreamCreateWithFlags(&g.s, cudaStreamNonBlocking));
+    CU(B.open());
     uint32_t *d_src, *hops, *ticket;
     float *dx, *dy;
     double *part, *d_out;
@@ -2407,15 +2462,15 @@ int gr_stress(uint32_t n, uint64_t m, const uint32_t *source, const uint32_t *ta
     if ((e = B.get(&d_src, k)) || (e = B.get(&hops, (size_t)k * n)) || (e = B.get(&dx, n)) || (e = B.get(&dy, n)) ||
         (e = B.get(&part, 3 * (size_t)G)) || (e = B.get(&d_out, 3)) || (e = B.get(&ticket, 1)))
         return set_err(GR_ALLOC_FAILED, cudaGetErrorString(e));
-    CU(cudaMemcpyAsync(d_src, from.data(), (size_t)k * 4, cudaMemcpyHostToDevice, g.s));
-    CU(cudaMemcpyAsync(dx, x, (size_t)n * 4, cudaMemcpyHostToDevice, g.s));
-    CU(cudaMemcpyAsync(dy, y, (size_t)n * 4, cudaMemcpyHostToDevice, g.s));
-    CU(cudaMemsetAsync(ticket, 0, 4, g.s));
-    if (int c = bfs_on_device(n, m, source, target, k, d_src, hops, g.s, B)) return c;
-    k_stress_sums<<<G, STRESS_T, 0, g.s>>>(n, k, d_src, hops, dx, dy, part, d_out, ticket);
+    CU(cudaMemcpyAsync(d_src, from.data(), (size_t)k * 4, cudaMemcpyHostToDevice, B.s));
+    CU(cudaMemcpyAsync(dx, x, (size_t)n * 4, cudaMemcpyHostToDevice, B.s));
+    CU(cudaMemcpyAsync(dy, y, (size_t)n * 4, cudaMemcpyHostToDevice, B.s));
+    CU(cudaMemsetAsync(ticket, 0, 4, B.s));
+    if (int c = bfs_on_device(n, m, source, target, k, d_src, hops, B)) return c;
+    k_stress_sums<<<G, STRESS_T, 0, B.s>>>(n, k, d_src, hops, dx, dy, part, d_out, ticket);
     double sums[3];
-    CU(cudaMemcpyAsync(sums, d_out, sizeof sums, cudaMemcpyDeviceToHost, g.s));
-    CU(cudaStreamSynchronize(g.s));
+    CU(cudaMemcpyAsync(sums, d_out, sizeof sums, cudaMemcpyDeviceToHost, B.s));
+    CU(cudaStreamSynchronize(B.s));
     const double de = sums[0], ee = sums[1], dd = sums[2];
     if (ee == 0.0 || dd == 0.0) return ok();
     *out = std::sqrt(std::max((dd - de / ee * de) / dd, 0.0));

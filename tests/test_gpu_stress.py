@@ -62,3 +62,18 @@ def test_refusals():
         S.bfs_hops(3, [0], [5], [0])  # endpoint out of range
     with pytest.raises(EngineError):
         S.bfs_hops(3, [0], [1], [3])  # source out of range
+
+
+@pytest.mark.parametrize("degree", [1, 63, 64, 65, 511, 512, 513, 6000])
+@pytest.mark.parametrize("tail", [0, 3, 4, 5, 9])
+def test_bfs_through_hubs_and_along_paths_equals_the_oracle(degree, tail):
+    """A hub whose row is summed by a lane or by the warp, several rounds of it, with a path behind its
+    first neighbour that ends before, at and past a round of levels; a stray node and a repeated edge."""
+    hub = np.zeros(degree, np.uint32)
+    leaves = np.arange(1, degree + 1, dtype=np.uint32)
+    path = np.concatenate([[1], degree + 1 + np.arange(tail)]).astype(np.uint32)
+    s = np.concatenate([hub, path[:-1], [0]]).astype(np.uint32)
+    d = np.concatenate([leaves, path[1:], [1]]).astype(np.uint32)
+    n = degree + tail + 2
+    src = np.unique(np.array([0, 1, degree, n - 2, n - 1], np.uint32))
+    assert np.array_equal(S.bfs_hops(n, s, d, src), O.bfs_hops(n, s, d, src))
