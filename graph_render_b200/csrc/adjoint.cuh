@@ -198,9 +198,15 @@ k_adj_node(uint32_t n, float gravity, int strong, const DevState *st, AdjScalars
 }
 
 // (3) The walk again, with the same decisions: for every far cell (and
-// one-point leaf) lam_i += J ub_i and the cell's centre adjoint -= J ub_i (one
-// FP64 atomic per warp and cell: the cell index is warp-uniform); for the pairs
-// of a several-point leaf the other point gets -J ub_i directly.
+// one-point leaf) lam_i += J ub_i and the cell's centre adjoint -= J ub_i, summed
+// over the ADJ_GROUP adjacent nodes that walk together (one FP64 atomic per group
+// and cell); for the pairs of a several-point leaf the other point gets -J ub_i
+// directly. A group's cell index is the same in its lanes, and the groups of a
+// warp step side by side: the union of eight nodes' walks is 40% shorter than the
+// union of 32, and the walk is one dependent load after another (a few warps an SM
+// at 50k nodes): 130 us with 32 nodes a group, 115 with eight.
+constexpr int ADJ_GROUP = 8;
+
 template <int D>
 __global__ void __launch_bounds__(WALK_THREADS)
 k_adj_walk(WalkParams P, const DevState *__restrict__ st, Cells cells, const float4 *__restrict__ sp,
@@ -212,6 +218,7 @@ k_adj_walk(WalkParams P, const DevState *__restrict__ st, Cells cells, const flo
     if (__all_sync(GR_FULL, p >= n)) return;
     const bool valid = p < n;
     const float4 me = valid ? sp[p] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const f2 xy = f2_pack(me.x, me.y);
     const uint32_t mylp = valid ? leaf_pre[uid[p]] : 0xffffffffu;
     const uint32_t oi = valid ? sorig[p] : 0u;
     float vx = 0.f, vy = 0.f, vz = 0.f;
@@ -224,69 +231,66 @@ k_adj_walk(WalkParams P, const DevState *__restrict__ st, Cells cells, const flo
     float lx = 0.f, ly = 0.f, lz = 0.f;
     const float kr = P.kr, th2 = P.theta2;
     const uint32_t lane = threadIdx.x % GR_WARP;
+    const uint32_t mine = ((1u << ADJ_GROUP) - 1u) << (lane & ~(uint32_t)(ADJ_GROUP - 1));  // this lane's group
     uint32_t k = 0;
-    while (k < ncells) {
-        CellRec<D> R = cell_rec<D, false>(cells, k);
-        if (cells.skip) R.skip = cells.skip[k];
-        const uint32_t skip = min(max(R.skip, k + 1), ncells);
+    while (__any_sync(GR_FULL, k < ncells)) {
+        const bool walking = k < ncells;
+        const uint32_t at = walking ? k : 0u;
+        CellRec<D> R = cell_rec<D, false>(cells, at);
+        if (cells.skip) R.skip = cells.skip[at];
+        const uint32_t skip = min(max(R.skip, at + 1), ncells);
         const bool one = R.w2 < 0.f, leaf = one || R.multi;
-        const float cm = R.m;
-        const bool active = resume <= k;
+        const bool active = walking && resume <= k;
         const bool holds = (k <= mylp) && (mylp < skip);
         float dx, dy, dz, d2;
-        cell_offset<D>(R, f2_pack(me.x, me.y), me.z, dx, dy, dz, d2);
+        cell_offset<D>(R, xy, me.z, dx, dy, dz, d2);
         const bool far = active && !holds && d2 > 0.f && fabsf(R.w2) < th2 * d2;
         const bool open = active && !far;
         // a one-point leaf's pair is its body term (the point is its own centre)
         const bool body = far || (one && open && !holds && d2 > 0.f);
         float jx = 0.f, jy = 0.f, jz = 0.f;
         if (body) {
-            rep_jac<D>(kr * me.w * cm, dx, dy, dz, vx, vy, vz, jx, jy, jz);
+            rep_jac<D>(kr * me.w * R.m, dx, dy, dz, vx, vy, vz, jx, jy, jz);
             lx += jx;
             ly += jy;
             lz += jz;
         }
         if (far) resume = skip;
-        const uint32_t any_body = __ballot_sync(GR_FULL, body);
-        if (any_body) {  // warp-aggregated centre adjoint of cell k
+        if (__any_sync(GR_FULL, body)) {  // the centre adjoint of each group's cell
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
+            for (int o = ADJ_GROUP / 2; o > 0; o >>= 1) {
                 jx += __shfl_xor_sync(GR_FULL, jx, o);
                 jy += __shfl_xor_sync(GR_FULL, jy, o);
                 if (D == 3) jz += __shfl_xor_sync(GR_FULL, jz, o);
             }
-            if (lane == 0) {
+            if ((lane % ADJ_GROUP) == 0 && walking && (jx != 0.f || jy != 0.f || jz != 0.f)) {
                 atomicAdd(&xbar[(size_t)k * D], -(double)jx);
                 atomicAdd(&xbar[(size_t)k * D + 1], -(double)jy);
                 if (D == 3) atomicAdd(&xbar[(size_t)k * D + 2], -(double)jz);
             }
         }
-        if (one) {
-            k = k + 1;
-        } else if (leaf) {
-            if (__any_sync(GR_FULL, open)) {
-                const uint2 range = __ldg(&cells.range[k]);
-                for (uint32_t jp = range.x; jp < min(range.y, n); jp++) {
-                    const float4 o = __ldg(&sp[jp]);
-                    if (open && jp != p) {
-                        const float ex = me.x - o.x, ey = me.y - o.y, ez = (D == 3) ? me.z - o.z : 0.f;
-                        if (!(ex == 0.f && ey == 0.f && (D == 2 || ez == 0.f))) {  // a jiggled pair is constant
-                            float ax, ay, az;
-                            rep_jac<D>(kr * me.w * o.w, ex, ey, ez, vx, vy, vz, ax, ay, az);
-                            lx += ax;
-                            ly += ay;
-                            lz += az;
-                            atomicAdd(&lam_pair[(size_t)jp * D], -(double)ax);
-                            atomicAdd(&lam_pair[(size_t)jp * D + 1], -(double)ay);
-                            if (D == 3) atomicAdd(&lam_pair[(size_t)jp * D + 2], -(double)az);
-                        }
+        const bool opens = (__ballot_sync(GR_FULL, open) & mine) != 0u;
+        if (R.multi && open) {
+            const uint2 range = __ldg(&cells.range[k]);
+            for (uint32_t jp = range.x; jp < min(range.y, n); jp++) {
+                const float4 o = __ldg(&sp[jp]);
+                if (jp != p) {
+                    const float ex = me.x - o.x, ey = me.y - o.y, ez = (D == 3) ? me.z - o.z : 0.f;
+                    if (!(ex == 0.f && ey == 0.f && (D == 2 || ez == 0.f))) {  // a jiggled pair is constant
+                        float ax, ay, az;
+                        rep_jac<D>(kr * me.w * o.w, ex, ey, ez, vx, vy, vz, ax, ay, az);
+                        lx += ax;
+                        ly += ay;
+                        lz += az;
+                        atomicAdd(&lam_pair[(size_t)jp * D], -(double)ax);
+                        atomicAdd(&lam_pair[(size_t)jp * D + 1], -(double)ay);
+                        if (D == 3) atomicAdd(&lam_pair[(size_t)jp * D + 2], -(double)az);
                     }
                 }
             }
-            k = k + 1;
-        } else {
-            k = __any_sync(GR_FULL, open) ? k + 1 : skip;
         }
+        __syncwarp();
+        if (walking) k = leaf || opens ? k + 1 : skip;
     }
     if (valid) {
         lam_rep[(size_t)oi * D] = lx;
@@ -331,7 +335,48 @@ __global__ void k_adj_down(const DevState *st, BinTree t, const uint32_t *__rest
 
 // (5) Attraction (CSR gather, state.rs:152-162 and networkx's linlog /
 // distributed_action), dL/dc per CSR entry, and the sum of every part into the
-// next lam.
+// next lam. A row of more than LIGHT_MAX entries is taken by the whole warp (a
+// hub's row in one lane's loop held up the tick: 12 ms at 400k power-law nodes).
+
+// CSR entry e of a row at p with ub / mass ai: its part of lam into acc, dL/dc
+// into gce.
+template <int D>
+__device__ __forceinline__ void adj_entry(uint32_t e, const double *pc, const double *ai, int lin_log, int dissuade,
+                                          const float4 *__restrict__ pos, const uint32_t *__restrict__ col,
+                                          const float *__restrict__ wt, const float *__restrict__ ub,
+                                          double *__restrict__ gce, double *acc) {
+    const uint32_t j = col[e];
+    const float4 q = pos[j];
+    const double qc[3] = {q.x, q.y, q.z};
+    double dl[3] = {0, 0, 0}, df[3] = {0, 0, 0};
+    for (int a = 0; a < D; a++) {
+        const double uj = (double)ub[(size_t)j * D + a];
+        dl[a] = qc[a] - pc[a];
+        df[a] = (dissuade ? uj / (double)q.w : uj) - ai[a];
+    }
+    const double c = wt[e];
+    double gi = 0.0;
+    if (lin_log) {
+        const double dist = sqrt(dl[0] * dl[0] + dl[1] * dl[1] + dl[2] * dl[2]);
+        double phi = 0.0, dphi = 0.0;
+        if (dist > 0.0) {
+            phi = log1p(dist) / dist;
+            dphi = (dist / (1.0 + dist) - log1p(dist)) / (dist * dist);
+        }
+        const double ddot = dl[0] * df[0] + dl[1] * df[1] + dl[2] * df[2];
+        for (int a = 0; a < D; a++) {
+            acc[a] += c * (phi * df[a] + (dist > 0.0 ? dphi * dl[a] * ddot / dist : 0.0));
+            gi += phi * ai[a] * dl[a];
+        }
+    } else {  // a linear pull: no length, no quotient
+        for (int a = 0; a < D; a++) {
+            acc[a] += c * df[a];
+            gi += ai[a] * dl[a];
+        }
+    }
+    gce[e] += gi;
+}
+
 template <int D>
 __global__ void __launch_bounds__(FRC_THREADS)
 k_adj_final(uint32_t n, int lin_log, int dissuade, const AdjScalars *A, const float4 *__restrict__ pos,
@@ -339,42 +384,43 @@ k_adj_final(uint32_t n, int lin_log, int dissuade, const AdjScalars *A, const fl
             const float *__restrict__ lam, const float *__restrict__ ub, const float *__restrict__ v,
             const float *__restrict__ lam_rep, const float *__restrict__ lam_com, double *__restrict__ gce,
             float *__restrict__ lam_out) {
-    const uint32_t i = blockIdx.x * FRC_THREADS + threadIdx.x;
-    if (i >= n) return;
-    const float4 p = pos[i];
-    const double pc[3] = {p.x, p.y, p.z};
-    double ai[3] = {0, 0, 0}, acc[3] = {0, 0, 0};
-    const double mi = dissuade ? (double)p.w : 1.0;
-    for (int a = 0; a < D; a++) ai[a] = ub[(size_t)i * D + a] / mi;
-    for (uint32_t e = rp[i]; e < rp[i + 1]; e++) {
-        const uint32_t j = col[e];
-        const float4 q = pos[j];
-        const double qc[3] = {q.x, q.y, q.z};
-        const double mj = dissuade ? (double)q.w : 1.0;
-        double dl[3] = {0, 0, 0}, df[3] = {0, 0, 0};
-        for (int a = 0; a < D; a++) {
-            dl[a] = qc[a] - pc[a];
-            df[a] = ub[(size_t)j * D + a] / mj - ai[a];
-        }
-        const double dist = sqrt(dl[0] * dl[0] + dl[1] * dl[1] + dl[2] * dl[2]);
-        double phi = 1.0, dphi = 0.0;
-        if (lin_log) {
-            if (dist > 0.0) {
-                phi = log1p(dist) / dist;
-                dphi = (dist / (1.0 + dist) - log1p(dist)) / (dist * dist);
-            } else {
-                phi = 0.0;
-            }
-        }
-        const double c = wt[e];
-        const double ddot = dl[0] * df[0] + dl[1] * df[1] + dl[2] * df[2];
-        double gi = 0.0;
-        for (int a = 0; a < D; a++) {
-            acc[a] += c * (phi * df[a] + (dist > 0.0 ? dphi * dl[a] * ddot / dist : 0.0));
-            gi += phi * ai[a] * dl[a];
-        }
-        gce[e] += gi;
+    const uint32_t i = blockIdx.x * FRC_THREADS + threadIdx.x, lane = threadIdx.x % GR_WARP;
+    if ((i & ~(GR_WARP - 1u)) >= n) return;  // whole warps only
+    const bool valid = i < n;
+    double pc[3] = {0, 0, 0}, ai[3] = {0, 0, 0}, acc[3] = {0, 0, 0};
+    uint32_t e0 = 0, e1 = 0;
+    if (valid) {
+        const float4 p = pos[i];
+        pc[0] = p.x;
+        pc[1] = p.y;
+        pc[2] = p.z;
+        const double mi = dissuade ? (double)p.w : 1.0;
+        for (int a = 0; a < D; a++) ai[a] = ub[(size_t)i * D + a] / mi;
+        e0 = rp[i];
+        e1 = rp[i + 1];
     }
+    const bool heavy = e1 - e0 > LIGHT_MAX;
+    if (!heavy)
+        for (uint32_t e = e0; e < e1; e++) adj_entry<D>(e, pc, ai, lin_log, dissuade, pos, col, wt, ub, gce, acc);
+    for (uint32_t rows = __ballot_sync(GR_FULL, heavy); rows; rows &= rows - 1) {
+        const int src = __ffs(rows) - 1;
+        const uint32_t r0 = __shfl_sync(GR_FULL, e0, src), r1 = __shfl_sync(GR_FULL, e1, src);
+        double rpc[3], rai[3], sum[3] = {0, 0, 0};
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            rpc[a] = __shfl_sync(GR_FULL, pc[a], src);
+            rai[a] = __shfl_sync(GR_FULL, ai[a], src);
+        }
+#pragma unroll 4
+        for (uint32_t e = r0 + lane; e < r1; e += GR_WARP)
+            adj_entry<D>(e, rpc, rai, lin_log, dissuade, pos, col, wt, ub, gce, sum);
+#pragma unroll
+        for (int a = 0; a < D; a++) {
+            const double t = warp_sum_d(sum[a]);
+            if ((int)lane == src) acc[a] = t;
+        }
+    }
+    if (!valid) return;
     for (int a = 0; a < D; a++) {
         const size_t k = (size_t)i * D + a;
         lam_out[k] = (float)((double)lam[k] + ((double)v[k] - A->vsum[a] / (double)n) + (double)lam_rep[k] +
@@ -419,6 +465,21 @@ __global__ void k_adj_rescale(uint32_t count, float *__restrict__ lam, uint64_t 
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += stride)
         lam[i] = ldexpf(lam[i], -k);
     for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < ne; e += stride) gce[e] = ldexp(gce[e], -k);
+}
+
+// The result: a carried value times 2^exponent (undoing k_adj_shift's scale; beyond
+// FP64's range it is not finite), in FP64; a
+// non-finite one sets *bad. in and out may be the same.
+template <typename T>
+__global__ void k_adj_result(uint64_t count, const T *in, double *out, const AdjScalars *A, uint32_t *bad) {
+    const long long x = A->exponent;
+    const int ex = (int)(x < -4096 ? -4096 : x > 4096 ? 4096 : x);
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += stride) {
+        const double v = ldexp((double)in[i], ex);
+        if (!isfinite(v)) *bad = 1u;
+        out[i] = v;
+    }
 }
 
 // dL/dc per simple edge (its two CSR entries), times dc/dw, onto the raw edge

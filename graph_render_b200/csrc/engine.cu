@@ -117,7 +117,7 @@ static int params_values(const uint8_t *bytes, size_t len, double *out) {
 // ------------------------------------------------------------- engine ------
 
 struct Adjoint;
-static void adjoint_release(Adjoint *a);
+static void adjoint_release(Adjoint *a, cudaStream_t s);
 
 struct gr_fa2 {
     int dim = 2;
@@ -182,6 +182,8 @@ struct gr_fa2 {
     cudaGraphExec_t texec = nullptr;
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     bool timing_events = false;  // set while the timed graph is captured
+    cudaGraph_t agraph = nullptr;  // the adjoint's tick, over the present record's buffers
+    cudaGraphExec_t aexec = nullptr;
     // the attraction branch of a captured tick: it forks after the tree build and
     // joins before the forces, beside the walk
     cudaStream_t aux = nullptr;
@@ -214,10 +216,17 @@ struct gr_fa2 {
         if (tgraph) cudaGraphDestroy(tgraph);
         texec = nullptr;
         tgraph = nullptr;
+        drop_adjoint_graph();
+    }
+    void drop_adjoint_graph() {
+        if (aexec) cudaGraphExecDestroy(aexec);
+        if (agraph) cudaGraphDestroy(agraph);
+        aexec = nullptr;
+        agraph = nullptr;
     }
     ~gr_fa2() {
-        if (adj) adjoint_release(adj);
         drop_graphs();
+        if (adj) adjoint_release(adj, stream);
         for (int i = 0; i < 4; i++)
             if (ev[i]) cudaEventDestroy(ev[i]);
         if (fork_ev) cudaEventDestroy(fork_ev);
@@ -1997,17 +2006,20 @@ struct Adjoint {
     double *lam_pair = nullptr, *xbar = nullptr, *gce = nullptr, *gs = nullptr, *graw = nullptr, *part = nullptr;
     AdjScalars *A = nullptr;
     DevState *before = nullptr;  // the state before the tick the captured adjoint tick differentiates
+    uint32_t *bad = nullptr;     // set when a gradient is not finite
+    // the handle's stream-ordered pool, like its own buffers
+    cudaStream_t stream = nullptr;
     std::vector<void *> allocs;
     template <typename T>
     cudaError_t alloc(T **p, size_t count) {
-        cudaError_t e = cudaMalloc((void **)p, (count ? count : 1) * sizeof(T));
+        cudaError_t e = cudaMallocAsync((void **)p, (count ? count : 1) * sizeof(T), stream);
         if (e == cudaSuccess) allocs.push_back((void *)*p);
         return e;
     }
 };
 
-static void adjoint_release(Adjoint *a) {
-    for (void *p : a->allocs) cudaFree(p);
+static void adjoint_release(Adjoint *a, cudaStream_t s) {
+    for (void *p : a->allocs) cudaFreeAsync(p, s);
     delete a;
 }
 
@@ -2057,9 +2069,10 @@ static void adjoint_tick(gr_fa2 *h, Adjoint *a, const DevState *before) {
                                                a->lam, a->ub, a->v, a->lam_rep, a->lam_com, a->gce, a->lam1);
 }
 
-// The adjoint tick captured once into a graph (its per-tick input, the state
-// before the tick, read from a->before); retried in plain stream order if the
-// capture with programmatic launches fails.
+// The adjoint tick captured into a graph (its per-tick input, the state before the
+// tick, read from a->before), kept until the record's buffers or the handle's
+// launches change; retried in plain stream order if the capture with programmatic
+// launches fails.
 static int capture_adjoint(gr_fa2 *h, Adjoint *a, cudaGraph_t *g, cudaGraphExec_t *x) {
     for (;;) {
         *g = nullptr;
@@ -2085,55 +2098,47 @@ static int capture_adjoint(gr_fa2 *h, Adjoint *a, cudaGraph_t *g, cudaGraphExec_
     }
 }
 
-// Destroys a captured graph when the scope ends.
-struct GraphGuard {
-    cudaGraph_t g = nullptr;
-    cudaGraphExec_t x = nullptr;
-    ~GraphGuard() {
-        if (x) cudaGraphExecDestroy(x);
-        if (g) cudaGraphDestroy(g);
-    }
-};
-
 extern "C" {
 
 int gr_fa2_adjoint_forward(gr_fa2 *h, uint32_t ticks, uint32_t every) {
     if (!h) return set_err(GR_INVALID_HANDLE, "null handle");
     if (every == 0) return set_err(GR_INVALID_ARGUMENT, "checkpoint interval must be >= 1");
-    if (h->adj) {
-        adjoint_release(h->adj);
-        h->adj = nullptr;
-    }
     const uint32_t n = h->n;
     const int D = h->dim;
-    Adjoint *a = new (std::nothrow) Adjoint();
-    if (!a) return set_err(GR_ALLOC_FAILED, "host allocation failed");
-    a->ticks = ticks;
-    a->every = every;
-    const uint32_t nck = ticks / every + 1;
-    const uint64_t ne = 2 * h->m;
     cudaError_t e;
-    if ((e = a->alloc(&a->ckpt, (size_t)nck * n)) || (e = a->alloc(&a->ckst, nck)) ||
-        (e = a->alloc(&a->segp, (size_t)every * n)) || (e = a->alloc(&a->segst, every)) ||
-        (e = a->alloc(&a->final_pos, n)) || (e = a->alloc(&a->final_st, 1)) ||
-        (e = a->alloc(&a->lam1, (size_t)n * D)) || (e = a->alloc(&a->lam, (size_t)n * D)) ||
-        (e = a->alloc(&a->ub, (size_t)n * D)) || (e = a->alloc(&a->v, (size_t)n * D)) ||
-        (e = a->alloc(&a->lam_rep, (size_t)n * D)) || (e = a->alloc(&a->lam_com, (size_t)n * D)) ||
-        (e = a->alloc(&a->lam_pair, (size_t)n * D)) || (e = a->alloc(&a->xbar, 2 * (size_t)n * D)) ||
-        (e = a->alloc(&a->gce, ne)) || (e = a->alloc(&a->gs, h->m)) || (e = a->alloc(&a->graw, h->m_raw)) ||
-        (e = a->alloc(&a->part, 3 * (size_t)div_up(n, FRC_THREADS) + 8)) || (e = a->alloc(&a->A, 1)) ||
-        (e = a->alloc(&a->before, 1))) {
-        adjoint_release(a);
-        return set_err(GR_ALLOC_FAILED, cudaGetErrorString(e));
-    }
-    if (!h->bt.cell_of) {
-        if ((e = h->alloc(&h->bt.cell_of, n))) {
-            adjoint_release(a);
+    Adjoint *a = h->adj;
+    if (!a || a->ticks != ticks || a->every != every) {  // the last record's buffers serve one of the same shape
+        if (a) {
+            h->drop_adjoint_graph();
+            adjoint_release(a, h->stream);
+            h->adj = nullptr;
+        }
+        if (!(a = new (std::nothrow) Adjoint())) return set_err(GR_ALLOC_FAILED, "host allocation failed");
+        a->stream = h->stream;
+        a->ticks = ticks;
+        a->every = every;
+        const uint32_t nck = ticks / every + 1;
+        const uint64_t ne = 2 * h->m;
+        if ((e = a->alloc(&a->ckpt, (size_t)nck * n)) || (e = a->alloc(&a->ckst, nck)) ||
+            (e = a->alloc(&a->segp, (size_t)every * n)) || (e = a->alloc(&a->segst, every)) ||
+            (e = a->alloc(&a->final_pos, n)) || (e = a->alloc(&a->final_st, 1)) ||
+            (e = a->alloc(&a->lam1, (size_t)n * D)) || (e = a->alloc(&a->lam, (size_t)n * D)) ||
+            (e = a->alloc(&a->ub, (size_t)n * D)) || (e = a->alloc(&a->v, (size_t)n * D)) ||
+            (e = a->alloc(&a->lam_rep, (size_t)n * D)) || (e = a->alloc(&a->lam_com, (size_t)n * D)) ||
+            (e = a->alloc(&a->lam_pair, (size_t)n * D)) || (e = a->alloc(&a->xbar, 2 * (size_t)n * D)) ||
+            (e = a->alloc(&a->gce, ne)) || (e = a->alloc(&a->gs, h->m)) || (e = a->alloc(&a->graw, h->m_raw)) ||
+            (e = a->alloc(&a->part, 3 * (size_t)div_up(n, FRC_THREADS) + 8)) || (e = a->alloc(&a->A, 1)) ||
+            (e = a->alloc(&a->before, 1)) || (e = a->alloc(&a->bad, 1))) {
+            adjoint_release(a, h->stream);
             return set_err(GR_ALLOC_FAILED, cudaGetErrorString(e));
         }
+        h->adj = a;
+    }
+    a->done = 0;
+    if (!h->bt.cell_of) {
+        if ((e = h->alloc(&h->bt.cell_of, n))) return set_err(GR_ALLOC_FAILED, cudaGetErrorString(e));
         h->drop_graphs();  // the captured tick now also records each cell's node
     }
-    h->adj = a;
     DevState s0;
     if (int c = read_state(h, &s0)) return c;
     if (n && ticks) {
@@ -2168,10 +2173,10 @@ int gr_fa2_adjoint_backward(gr_fa2 *h, const float *dL_dpT, double *dL_dp0, doub
     CU(cudaMemcpyAsync(a->lam1, dL_dpT, (size_t)n * D * 4, cudaMemcpyHostToDevice, s));
     CU(cudaMemsetAsync(a->A, 0, sizeof(AdjScalars), s));
     CU(cudaMemsetAsync(a->gce, 0, std::max<uint64_t>(2 * h->m, 1) * sizeof(double), s));
-    GraphGuard adj;  // the adjoint tick, captured once per call
     if (n && a->done) {
         if (int c = build_graph(h)) return c;  // the replay runs the recorded run's own tick graph
-        if (int c = capture_adjoint(h, a, &adj.g, &adj.x)) return c;
+        if (!h->aexec)
+            if (int c = capture_adjoint(h, a, &h->agraph, &h->aexec)) return c;
         const uint32_t nseg = (a->done + a->every - 1) / a->every;
         for (uint32_t g = nseg; g-- > 0;) {
             const uint32_t t0 = g * a->every, t1 = std::min(t0 + a->every, a->done);
@@ -2188,15 +2193,18 @@ int gr_fa2_adjoint_backward(gr_fa2 *h, const float *dL_dpT, double *dL_dp0, doub
                                    cudaMemcpyDeviceToDevice, s));
                 CU(cudaMemcpyAsync(h->st, a->segst + (t - t0), sizeof(DevState), cudaMemcpyDeviceToDevice, s));
                 CU(cudaMemcpyAsync(a->before, a->segst + (t - t0), sizeof(DevState), cudaMemcpyDeviceToDevice, s));
-                CU(cudaGraphLaunch(adj.x, s));
+                CU(cudaGraphLaunch(h->aexec, s));
             }
         }
     }
     CU(cudaGetLastError());
-    std::vector<float> lam0((size_t)n * D);
-    AdjScalars Ah;
-    if (n) CU(cudaMemcpyAsync(lam0.data(), a->lam1, (size_t)n * D * 4, cudaMemcpyDeviceToHost, s));
-    CU(cudaMemcpyAsync(&Ah, a->A, sizeof(AdjScalars), cudaMemcpyDeviceToHost, s));
+    CU(cudaMemsetAsync(a->bad, 0, 4, s));
+    const auto result_blocks = [](uint64_t count) { return (uint32_t)std::min<uint64_t>((count + 255) / 256, 4 * 148); };
+    if (n) {  // into xbar, which the ticks are done with
+        const uint64_t count = (uint64_t)n * D;
+        k_adj_result<float><<<result_blocks(count), 256, 0, s>>>(count, a->lam1, a->xbar, a->A, a->bad);
+        CU(cudaMemcpyAsync(dL_dp0, a->xbar, count * sizeof(double), cudaMemcpyDeviceToHost, s));
+    }
     if (dL_dw && h->m_raw) {
         CU(cudaMemsetAsync(a->gs, 0, std::max<uint64_t>(h->m, 1) * sizeof(double), s));
         CU(cudaMemsetAsync(a->graw, 0, h->m_raw * sizeof(double), s));
@@ -2204,23 +2212,16 @@ int gr_fa2_adjoint_backward(gr_fa2 *h, const float *dL_dpT, double *dL_dp0, doub
             k_adj_edges<<<div_up(2 * h->m, 256), 256, 0, s>>>((uint32_t)(2 * h->m), h->csr_simple, a->gce, a->gs);
             k_adj_raw<<<div_up(h->m, 256), 256, 0, s>>>((uint32_t)h->m, a->gs, h->simple_raw, h->simple_dcdw, a->graw);
         }
+        k_adj_result<double><<<result_blocks(h->m_raw), 256, 0, s>>>(h->m_raw, a->graw, a->graw, a->A, a->bad);
         CU(cudaMemcpyAsync(dL_dw, a->graw, h->m_raw * sizeof(double), cudaMemcpyDeviceToHost, s));
     }
+    uint32_t bad = 0;
+    CU(cudaMemcpyAsync(&bad, a->bad, 4, cudaMemcpyDeviceToHost, s));
     // the handle goes back to the end of the recorded run
     CU(cudaMemcpyAsync(h->pos, a->final_pos, (size_t)std::max(n, 1u) * sizeof(float4), cudaMemcpyDeviceToDevice, s));
     CU(cudaMemcpyAsync(h->st, a->final_st, sizeof(DevState), cudaMemcpyDeviceToDevice, s));
     CU(cudaStreamSynchronize(s));
-    // undo the running power-of-two scale (k_adj_shift); beyond FP64's range is non-finite
-    const int ex = (int)std::max<long long>(-4096, std::min<long long>(4096, Ah.exponent));
-    for (size_t i = 0; i < (size_t)n * D; i++) {
-        dL_dp0[i] = std::ldexp((double)lam0[i], ex);
-        if (!std::isfinite(dL_dp0[i])) return set_err(GR_LAYOUT_FAILED, "non-finite gradient");
-    }
-    if (dL_dw)
-        for (uint64_t e = 0; e < h->m_raw; e++) {
-            dL_dw[e] = std::ldexp(dL_dw[e], ex);
-            if (!std::isfinite(dL_dw[e])) return set_err(GR_LAYOUT_FAILED, "non-finite gradient");
-        }
+    if (bad) return set_err(GR_LAYOUT_FAILED, "non-finite gradient");
     return ok();
 }
 

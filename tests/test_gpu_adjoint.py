@@ -181,3 +181,43 @@ def test_backward_seeded_with_the_stress_loss_matches_the_oracle(theta, ticks):
     op, ow = oracle_grad(wl, w, prm, ticks, g, dense=(theta == 0.0))
     assert rel(gp, op) < TOL, rel(gp, op)
     assert rel(gw, ow) < TOL, rel(gw, ow)
+
+
+@pytest.mark.parametrize("opts", [{}, dict(lin_log=1, dissuade_hubs=1)], ids=["linear", "linlog"])
+@pytest.mark.parametrize("degree", [63, 64, 65, 640])
+def test_rows_either_side_of_the_warps_limit_match_the_oracle(degree, opts):
+    """A hub whose row is summed by one lane or by the warp, one tick, to the file's tolerance."""
+    n = 700
+    rng = np.random.default_rng(degree)
+    s = np.concatenate([np.zeros(degree), np.arange(1, n - 1)]).astype(np.uint32)
+    d = np.concatenate([np.arange(1, degree + 1), np.arange(2, n)]).astype(np.uint32)
+    wl = synth.Workload("hub", n, s, d, None, rng.uniform(-300, 300, (n, 2)).astype(np.float32),
+                        dict(theta=1.2, dim=2, seed=3, max_iter=1, edge_weight_influence=1.0, **opts), 1)
+    w = rng.uniform(0.5, 1.5, wl.m)
+    R = rng.normal(size=(n, 2))
+    gp, gw = gpu_grad(wl, w, wl.params, 1, R)
+    op, ow = oracle_grad(wl, w, wl.params, 1, R, dense=False)
+    assert rel(gp, op) < TOL and rel(gw, ow) < TOL, (rel(gp, op), rel(gw, ow))
+
+
+def test_a_record_over_the_last_ones_buffers_gives_a_fresh_handles_gradient():
+    """Records of one shape share buffers and the captured adjoint tick; another schedule or shape drops
+    them. Atomic sums of FP64 terms may land in another order: 1e-6 covers their FP32 rounding."""
+    wl, w, prm = instance(n=3000, theta=1.2)
+    R = np.random.default_rng(9).normal(size=(wl.n, 2))
+    moved = wl.pos0 + np.random.default_rng(10).normal(size=wl.pos0.shape).astype(np.float32)
+    with Fa2(wl.n, wl.src, wl.dst, w, params=prm, pos0=wl.pos0) as eng:
+        eng.adjoint_forward(1, 1)
+        eng.adjoint_backward(R)
+        for step in ("same shape", "another schedule", "another shape", "that shape again"):
+            ticks, every = (1, 1) if step in ("same shape", "another schedule") else (2, 1)
+            if step == "another schedule":
+                eng.set_walk_schedule(2)
+            eng.set_positions(moved)
+            eng.set_controller(1.0, 1.0, 1.0, 1.0, 0)
+            eng.adjoint_forward(ticks, every)
+            gp, gw = eng.adjoint_backward(R)
+            with Fa2(wl.n, wl.src, wl.dst, w, params=prm, pos0=moved) as fresh:
+                fresh.adjoint_forward(ticks, every)
+                fp, fw = fresh.adjoint_backward(R)
+            assert rel(gp, fp) < 1e-6 and rel(gw, fw) < 1e-6, (step, rel(gp, fp), rel(gw, fw))
