@@ -501,7 +501,6 @@ __global__ void __launch_bounds__(BT, BatchOcc<BT>::MIN_BLOCKS) k_batch(BatchArg
             __syncthreads();
             const uint32_t ncells = block_scan_excl<BT>(S.excl, S.P, nu, s_warp);
             {
-                constexpr int L = Levels<D>::L;
                 for (uint32_t s = t; s < nu; s += BT) {  // leaf cells
                     const uint32_t idx = S.P[s] + (uint32_t)__popc(S.levels[s]);
                     const uint32_t a0 = S.leaf_start[s], a1 = S.leaf_start[s + 1];
@@ -509,12 +508,8 @@ __global__ void __launch_bounds__(BT, BatchOcc<BT>::MIN_BLOCKS) k_batch(BatchArg
                         atomicOr(&s_st.error, (uint32_t)ERR_TREE);
                         continue;
                     }
-                    const float4 one = S.sp[a0];
-                    bool coinc;
-                    const Body body = leaf_sum<D>(S.sp, a0, a1, coinc);
-                    const int level = nu == 1 ? 0 : coinc ? S.bt.delta[S.bt.leaf_parent[s]] / D + 1 : L;
-                    write_cell<D>(S.cells, idx, body, level, s_root_w, idx + 1, a0, a1 - a0,
-                                  a1 - a0 == 1 ? &one : nullptr);
+                    write_leaf<D>(S.cells, idx, S.sp, a0, a1, s_root_w, nu == 1,
+                                  [&] { return S.bt.delta[S.bt.leaf_parent[s]]; });
                     S.leaf_pre[s] = idx;
                 }
                 for (uint32_t i = t; i + 1 < nu; i += BT) {  // internal cells

@@ -122,6 +122,31 @@ __device__ __forceinline__ double block_sum_d(double v, double *smem) {
     return r;
 }
 
+// K such sums at once, each the same bits as block_sum_d's. One at a time, K sums
+// are K chains of ten FP64 shuffles and two barriers, most of a small grid's last
+// block; together their shuffles overlap and share the barriers.
+template <int THREADS, int K>
+__device__ __forceinline__ void block_sums_d(double *v, double (*smem)[K]) {
+    const int w = threadIdx.x / GR_WARP, l = threadIdx.x % GR_WARP;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < K; k++) v[k] += __shfl_xor_sync(GR_FULL, v[k], o);
+    if (l == 0)
+#pragma unroll
+        for (int k = 0; k < K; k++) smem[w][k] = v[k];
+    __syncthreads();
+    if (w == 0) {
+#pragma unroll
+        for (int k = 0; k < K; k++) v[k] = l < THREADS / GR_WARP ? smem[l][k] : 0.0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int k = 0; k < K; k++) v[k] += __shfl_xor_sync(GR_FULL, v[k], o);
+    }
+    __syncthreads();
+}
+
 // Sum of v[k * stride + off] over this thread's k = threadIdx.x, threadIdx.x +
 // T, ... < count, added in k order; U loads are in flight at a time (the same
 // sum as one load per step, without a round trip per step).
@@ -145,15 +170,17 @@ __device__ __forceinline__ double strided_sum_cg(const double *v, uint32_t count
 // True in exactly one thread of the grid's last block to finish (threadfence
 // reduction pattern); the ticket resets itself for the next launch.
 __device__ __forceinline__ bool last_block_done(uint32_t *ticket, bool *smem_flag) {
-    __threadfence();
+    // one thread's fences order the whole block's accesses: the barriers put the
+    // other threads' before the first and after the second
     __syncthreads();
     if (threadIdx.x == 0) {
+        __threadfence();
         uint32_t t = atomicAdd(ticket, 1u);
         *smem_flag = (t == gridDim.x - 1);
         if (*smem_flag) *ticket = 0;
+        __threadfence();
     }
     __syncthreads();
-    if (*smem_flag) __threadfence();
     return *smem_flag;
 }
 

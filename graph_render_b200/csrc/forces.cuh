@@ -371,9 +371,9 @@ k_forces(ForceParams P, DevState *st, const float4 *__restrict__ pos, const floa
          double *__restrict__ part, int speed_update) {
     gr_pdl_enter();
     if (st->converged) return;
-    __shared__ double s_red[32];
+    __shared__ double s_red[FRC_THREADS / GR_WARP][2];
     __shared__ bool s_last;
-    double sw = 0.0, tr = 0.0;
+    double sum[2] = {0.0, 0.0};  // swing, traction
     const double mean[3] = {st->mean[0], st->mean[1], st->mean[2]};
     for (uint32_t i = blockIdx.x * FRC_THREADS + threadIdx.x; i < P.n; i += gridDim.x * FRC_THREADS) {
         const float4 p = pos[i];
@@ -382,33 +382,35 @@ k_forces(ForceParams P, DevState *st, const float4 *__restrict__ pos, const floa
         double s1, t1;
         node_force<D>(P, p, a0, a1, a2, rep[(size_t)i * D + 0], rep[(size_t)i * D + 1],
                       D == 3 ? rep[(size_t)i * D + 2] : 0.f, mean, u, s1, t1);
-        sw += s1;
-        tr += t1;
+        sum[0] += s1;
+        sum[1] += t1;
     }
     if (!speed_update) return;
-    sw = block_sum_d<FRC_THREADS>(sw, s_red);
-    tr = block_sum_d<FRC_THREADS>(tr, s_red);
+    block_sums_d<FRC_THREADS, 2>(sum, s_red);
     if (threadIdx.x == 0) {
-        part[2 * blockIdx.x] = sw;
-        part[2 * blockIdx.x + 1] = tr;
+        part[2 * blockIdx.x] = sum[0];
+        part[2 * blockIdx.x + 1] = sum[1];
     }
     if (!last_block_done(&st->counters[1], &s_last)) return;
-    double a = strided_sum_cg<FRC_THREADS>(part, gridDim.x, 2, 0);
-    double b = strided_sum_cg<FRC_THREADS>(part, gridDim.x, 2, 1);
-    a = block_sum_d<FRC_THREADS>(a, s_red);
-    b = block_sum_d<FRC_THREADS>(b, s_red);
+    sum[0] = strided_sum_cg<FRC_THREADS>(part, gridDim.x, 2, 0);
+    sum[1] = strided_sum_cg<FRC_THREADS>(part, gridDim.x, 2, 1);
+    block_sums_d<FRC_THREADS, 2>(sum, s_red);
     if (threadIdx.x == 0) {
-        st->swing += a;
-        st->traction += b;
+        st->swing += sum[0];
+        st->traction += sum[1];
         estimate_factor(st, (double)P.n, P.jitter_tolerance);
     }
 }
 
 // The update for every node; FP64 sum of |step| decides the 1e-10 early exit
-// (state.rs:122-128). With bpart, the same pass also takes the new positions'
+// (state.rs:122-128). The same pass also takes the new positions'
 // extent and FP64 sums (bounds_block / bounds_finish over k_bounds' grid and
 // per-thread order, so the same bits k_bounds would get) into the root square
 // and mean of the next tick, and stamps them valid for it.
+// On a small grid both this pass and k_forces are the latency of their reductions:
+// sums taken together, extents by warp shuffles, one fence a block and a root
+// square that starts near its size took a 1,500-node tick from 70.4 to 63.3 us with
+// the leaf prefix's shorter folds (100,000 nodes: 158 to 151; same bits).
 static_assert(FRC_THREADS == BND_THREADS, "k_update and k_bounds share one grid shape");
 template <int D>
 __global__ void __launch_bounds__(FRC_THREADS)
@@ -416,14 +418,14 @@ k_update(uint32_t n, DevState *st, float4 *__restrict__ pos, const float *__rest
          double *__restrict__ part, double *__restrict__ bpart) {
     gr_pdl_enter();
     if (st->converged) return;
-    __shared__ double s_red[32];
-    __shared__ float s_f[2 * D][32];
+    __shared__ double s_red[BND_W][D + 1], s_g[2 * D][BND_W];
+    __shared__ float s_f[2 * D][BND_W];
     __shared__ bool s_last;
-    double step = 0.0;
+    double sum[D + 1];  // the new positions', then the steps'
     bool bad = false;
     const double speed = st->speed;
     float lo[D], hi[D];
-    double sum[D];
+    sum[D] = 0.0;
 #pragma unroll
     for (int a = 0; a < D; a++) {
         lo[a] = INFINITY;
@@ -433,7 +435,7 @@ k_update(uint32_t n, DevState *st, float4 *__restrict__ pos, const float *__rest
     for (uint32_t i = blockIdx.x * FRC_THREADS + threadIdx.x; i < n; i += gridDim.x * FRC_THREADS) {
         float4 p = pos[i];
         bool b;
-        step += node_update<D>(p, U + (size_t)i * D, speed, b);
+        sum[D] += node_update<D>(p, U + (size_t)i * D, speed, b);
         bad = bad || b;
         pos[i] = p;
         const float c[3] = {p.x, p.y, p.z};
@@ -445,20 +447,16 @@ k_update(uint32_t n, DevState *st, float4 *__restrict__ pos, const float *__rest
         }
     }
     if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(&st->error, (uint32_t)ERR_NONFINITE);
-    if (bpart) bounds_block<D>(lo, hi, sum, bpart, s_red, s_f);
-    step = block_sum_d<FRC_THREADS>(step, s_red);
-    if (threadIdx.x == 0) part[blockIdx.x] = step;
+    bounds_block<D, D + 1>(lo, hi, sum, bpart, s_red, s_f);
+    if (threadIdx.x == 0) part[blockIdx.x] = sum[D];
     if (!last_block_done(&st->counters[2], &s_last)) return;
-    double a = strided_sum_cg<FRC_THREADS>(part, gridDim.x, 1, 0);
-    a = block_sum_d<FRC_THREADS>(a, s_red);
+    sum[D] = strided_sum_cg<FRC_THREADS>(part, gridDim.x, 1, 0);
+    bounds_finish<D, D + 1>(bpart, n, st, sum, s_red, s_g);
     if (threadIdx.x == 0) {
-        st->moved = a;
+        st->moved = sum[D];
         st->iter_no += 1;
-        if (a < 1e-10 || st->error) st->converged = 1;
-    }
-    if (bpart) {
-        bounds_finish<D>(bpart, n, st, s_red);
-        if (threadIdx.x == 0) st->bounds_stamp = st->iter_no + 1u;
+        if (sum[D] < 1e-10 || st->error) st->converged = 1;
+        st->bounds_stamp = st->iter_no + 1u;
     }
 }
 

@@ -73,7 +73,14 @@ template <int D>
 __device__ __forceinline__ double root_square(const double *mn, const double *mx, double *root0, bool &ok) {
     double z = 1.0;
     ok = true;
-    for (int a = 0; a < D; a++) root0[a] = floor(mn[a]);
+    double widest = 0.0;
+    for (int a = 0; a < D; a++) {
+        root0[a] = floor(mn[a]);
+        widest = fmax(widest, mx[a] - root0[a]);
+    }
+    // Every power of two up to half the widest side is too small, whatever the
+    // sums' rounding: the doubling starts there, not at 1 (it runs in one thread).
+    if (widest >= 4.0 && isfinite(widest)) z = ldexp(1.0, ilogb(widest) - 1);
     for (bool grow = true; grow;) {
         grow = false;
         for (int a = 0; a < D; a++)
@@ -130,56 +137,72 @@ struct ZeroWords {
     }
 };
 
-// A block's extent and FP64 coordinate sums of this thread's positions (lo, hi,
-// sum, accumulated over its strided nodes in order): warp shuffles for min / max,
-// block_sum_d for the sums, one record of 3 D doubles per block in part.
-template <int D>
-__device__ __forceinline__ void bounds_block(const float *lo, const float *hi, const double *sum,
-                                             double *__restrict__ part, double *s_red, float (*s_f)[32]) {
+constexpr int BND_W = BND_THREADS / GR_WARP;
+
+// The minimum of lo and the maximum of hi over the block, per axis (exact in any
+// order), in every thread of warp 0. s_f: 2 D x BND_W.
+template <int D, typename T>
+__device__ __forceinline__ void block_extent(T *lo, T *hi, T (*s_f)[BND_W]) {
     const int lane = threadIdx.x % GR_WARP, w = threadIdx.x / GR_WARP;
+    auto fold = [&](int from) {
 #pragma unroll
-    for (int a = 0; a < D; a++) {
-        float l = lo[a], h = hi[a];
+        for (int o = from; o > 0; o >>= 1)
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            l = fminf(l, __shfl_xor_sync(GR_FULL, l, o));
-            h = fmaxf(h, __shfl_xor_sync(GR_FULL, h, o));
+            for (int a = 0; a < D; a++) {
+                lo[a] = min(lo[a], __shfl_xor_sync(GR_FULL, lo[a], o));
+                hi[a] = max(hi[a], __shfl_xor_sync(GR_FULL, hi[a], o));
+            }
+    };
+    fold(16);
+    if (lane == 0)
+#pragma unroll
+        for (int a = 0; a < D; a++) {
+            s_f[a][w] = lo[a];
+            s_f[D + a][w] = hi[a];
         }
-        if (lane == 0) {
-            s_f[a][w] = l;
-            s_f[D + a][w] = h;
+    __syncthreads();
+    if (w == 0) {
+#pragma unroll
+        for (int a = 0; a < D; a++) {
+            lo[a] = s_f[a][lane % BND_W];
+            hi[a] = s_f[D + a][lane % BND_W];
         }
+        fold(BND_W / 2);
     }
-    double tot[D];
-#pragma unroll
-    for (int a = 0; a < D; a++) tot[a] = block_sum_d<BND_THREADS>(sum[a], s_red);
+}
+
+// A block's extent and FP64 coordinate sums of this thread's positions (lo, hi and
+// v[0 .. D), accumulated over its strided nodes in order), one record of 3 D
+// doubles per block in part; v's other K - D sums are the caller's, in thread 0.
+template <int D, int K>
+__device__ __forceinline__ void bounds_block(float *lo, float *hi, double *v, double *__restrict__ part,
+                                             double (*s_red)[K], float (*s_f)[BND_W]) {
+    block_extent<D>(lo, hi, s_f);
+    block_sums_d<BND_THREADS, K>(v, s_red);
     if (threadIdx.x == 0) {
         double *q = part + (size_t)blockIdx.x * 3 * D;
+#pragma unroll
         for (int a = 0; a < D; a++) {
-            float l = INFINITY, h = -INFINITY;
-            for (int k = 0; k < BND_THREADS / GR_WARP; k++) {
-                l = fminf(l, s_f[a][k]);
-                h = fmaxf(h, s_f[D + a][k]);
-            }
-            q[a] = l;
-            q[D + a] = h;
-            q[2 * D + a] = tot[a];
+            q[a] = lo[a];
+            q[D + a] = hi[a];
+            q[2 * D + a] = v[a];
         }
     }
 }
 
 // The grid's last block: the block records folded in block order into the
 // reference's root square (quadtree.rs:157-195 cover, both corners) and the
-// mean gravity pulls toward (state.rs:208-218).
-template <int D>
-__device__ __forceinline__ void bounds_finish(const double *part, uint32_t n, DevState *st, double *s_red) {
-    const int lane = threadIdx.x % GR_WARP, w = threadIdx.x / GR_WARP;
-    double gl[D], gh[D], gs[D];
+// mean gravity pulls toward (state.rs:208-218). v[D .. K) are the caller's sums
+// over threads, folded beside; in thread 0 afterwards.
+template <int D, int K>
+__device__ __forceinline__ void bounds_finish(const double *part, uint32_t n, DevState *st, double *v,
+                                              double (*s_red)[K], double (*s_f)[BND_W]) {
+    double gl[D], gh[D];
 #pragma unroll
     for (int a = 0; a < D; a++) {
         gl[a] = INFINITY;
         gh[a] = -INFINITY;
-        gs[a] = 0.0;
+        v[a] = 0.0;
     }
     for (uint32_t b = threadIdx.x; b < gridDim.x; b += BND_THREADS) {
         const double *q = part + (size_t)b * 3 * D;
@@ -187,42 +210,17 @@ __device__ __forceinline__ void bounds_finish(const double *part, uint32_t n, De
         for (int a = 0; a < D; a++) {
             gl[a] = fmin(gl[a], __ldcg(q + a));
             gh[a] = fmax(gh[a], __ldcg(q + D + a));
-            gs[a] += __ldcg(q + 2 * D + a);
+            v[a] += __ldcg(q + 2 * D + a);
         }
     }
-    // min / max are exact in any order: warp shuffles, then the warp results
-    __shared__ double s_l[D][BND_THREADS / GR_WARP], s_h[D][BND_THREADS / GR_WARP];
-#pragma unroll
-    for (int a = 0; a < D; a++) {
-        double l = gl[a], h = gh[a];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            l = fmin(l, __shfl_xor_sync(GR_FULL, l, o));
-            h = fmax(h, __shfl_xor_sync(GR_FULL, h, o));
-        }
-        if (lane == 0) {
-            s_l[a][w] = l;
-            s_h[a][w] = h;
-        }
-    }
-    double S[D];
-#pragma unroll
-    for (int a = 0; a < D; a++) S[a] = block_sum_d<BND_THREADS>(gs[a], s_red);
+    block_extent<D>(gl, gh, s_f);
+    block_sums_d<BND_THREADS, K>(v, s_red);
     if (threadIdx.x == 0) {
-        double mn[D], mx[D];
-        for (int a = 0; a < D; a++) {
-            mn[a] = INFINITY;
-            mx[a] = -INFINITY;
-            for (int k = 0; k < BND_THREADS / GR_WARP; k++) {
-                mn[a] = fmin(mn[a], s_l[a][k]);
-                mx[a] = fmax(mx[a], s_h[a][k]);
-            }
-        }
         bool ok = true;
-        const double z = root_square<D>(mn, mx, st->root0, ok);
+        const double z = root_square<D>(gl, gh, st->root0, ok);
         if (!ok) atomicOr(&st->error, (uint32_t)ERR_BOUNDS);
         st->root_w = z;
-        for (int a = 0; a < D; a++) st->mean[a] = S[a] / (double)n;
+        for (int a = 0; a < D; a++) st->mean[a] = v[a] / (double)n;
         if (st->error) st->converged = 1;
     }
 }
@@ -239,8 +237,8 @@ k_bounds(const float4 *__restrict__ pos, uint32_t n, DevState *st, double *__res
     if (st->converged) return;
     if (blockIdx.x == 0) zw.clear();
     if (st->bounds_stamp == st->iter_no + 1u) return;
-    __shared__ double s_red[32];
-    __shared__ float s_f[2 * D][32];
+    __shared__ double s_red[BND_W][D], s_g[2 * D][BND_W];
+    __shared__ float s_f[2 * D][BND_W];
     __shared__ bool s_last;
     float lo[D], hi[D];
     double sum[D];
@@ -277,9 +275,9 @@ k_bounds(const float4 *__restrict__ pos, uint32_t n, DevState *st, double *__res
     if (__syncthreads_or(bad)) {
         if (threadIdx.x == 0) atomicOr(&st->error, (uint32_t)ERR_NONFINITE);
     }
-    bounds_block<D>(lo, hi, sum, part, s_red, s_f);
+    bounds_block<D, D>(lo, hi, sum, part, s_red, s_f);
     if (!last_block_done(&st->counters[0], &s_last)) return;
-    bounds_finish<D>(part, n, st, s_red);
+    bounds_finish<D, D>(part, n, st, sum, s_red, s_g);
 }
 
 // Morton key of every node in the root square: per axis q = floor((x - x0) *
@@ -753,7 +751,9 @@ constexpr uint32_t LEAF_FOLD_MAX_TILES = 2048;
 // leaves they start, folded by the calling block (AG_T threads) in a fixed
 // shape: thread t adds tiles t, t + AG_T, ... < b in turn, the lanes of a warp
 // combine by a shuffle-down tree into lane 0, and one thread adds the warp
-// totals in warp order. s_bw / s_bc hold AG_W + 1 entries.
+// totals in warp order. A lane or a warp that had no tile holds zeros, whose
+// addition changes nothing and is left out: a double-double addition is a chain
+// of dependent FP64 operations. s_bw / s_bc hold AG_W + 1 entries.
 template <int D>
 __device__ __forceinline__ void tiles_before(uint32_t b, const Body *__restrict__ tile_sum,
                                              const uint32_t *__restrict__ tile_cnt, BodyDD &carry, uint32_t &count,
@@ -780,6 +780,7 @@ __device__ __forceinline__ void tiles_before(uint32_t b, const Body *__restrict_
     const int lane = threadIdx.x % GR_WARP, w = threadIdx.x / GR_WARP;
 #pragma unroll
     for (int o = GR_WARP / 2; o >= 1; o >>= 1) {
+        if (w * GR_WARP + o >= (int)b) continue;  // the upper lanes of this step had no tile
         const BodyDD u = bdd_shfl_down<D>(acc, o);
         const uint32_t cu = __shfl_down_sync(GR_FULL, c, o);
         if (lane < o) {
@@ -795,7 +796,8 @@ __device__ __forceinline__ void tiles_before(uint32_t b, const Body *__restrict_
     if (threadIdx.x == 0) {
         BodyDD t = s_bw[0];
         uint32_t tc = s_bc[0];
-        for (int q = 1; q < AG_W; q++) {
+        const int held = min(((int)b + GR_WARP - 1) / GR_WARP, AG_W);  // b is at most LEAF_FOLD_MAX_TILES
+        for (int q = 1; q < held; q++) {
             t = bdd_add<D>(t, s_bw[q]);
             tc += s_bc[q];
         }
@@ -1034,27 +1036,19 @@ __device__ __forceinline__ CellRec<D> cell_rec(const Cells &c, uint32_t k) {
     return r;
 }
 
-// leaf: 0 for an internal cell, else its point count.
+// The exponent field, in place, of the FP32 value of w^2 at a level: w is root_w / 2^level.
+__device__ __forceinline__ uint32_t cell_w2(double root_w, int level) {
+    const int e = 2 * ((int)((__double2hiint(root_w) >> 20) & 0x7ff) - 1023 - level) + 127;
+    return (uint32_t)min(max(e, 0), 255) << 23;
+}
+
+// The record of a cell with centre hi + lo and mass m. leaf: 0 for an internal
+// cell, else its point count.
 template <int D>
-__device__ __forceinline__ void write_cell(Cells c, uint32_t idx, const Body &b, int level, double root_w,
-                                           uint32_t skip, uint32_t start, uint32_t leaf, const float4 *point = nullptr) {
-    double inv = 1.0 / b.m;
-    double cc[3] = {b.c0 * inv, b.c1 * inv, b.c2 * inv};
-    if (point) {  // a one-point leaf's centre is the point itself, exactly
-        cc[0] = point->x;
-        cc[1] = point->y;
-        cc[2] = point->z;
-    }
-    float hi[3], lo[3];
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-        hi[a] = (float)cc[a];
-        lo[a] = (float)(cc[a] - (double)hi[a]);
-    }
-    const double w = ldexp(root_w, -level);
-    const uint32_t word = (__float_as_uint((float)(w * w)) & 0x7f800000u) | (leaf == 1 ? 0x80000000u : 0u) |
-                          (leaf > 1 ? CELL_MULTI : 0u) | (c.skip ? 0u : skip & CELL_SKIP);
-    const float m = (float)b.m;
+__device__ __forceinline__ void put_cell(const Cells &c, uint32_t idx, const float *hi, const float *lo, float m,
+                                         int level, double root_w, uint32_t skip, uint32_t start, uint32_t leaf) {
+    const uint32_t word = cell_w2(root_w, level) | (leaf == 1 ? 0x80000000u : 0u) | (leaf > 1 ? CELL_MULTI : 0u) |
+                          (c.skip ? 0u : skip & CELL_SKIP);
     if (D == 2) {
         c.a[idx] = make_float4(-hi[0], -hi[1], -lo[0], -lo[1]);
         c.b[idx] = make_float2(m, __uint_as_float(word));
@@ -1065,6 +1059,39 @@ __device__ __forceinline__ void write_cell(Cells c, uint32_t idx, const Body &b,
     if (leaf > 1) c.range[idx] = make_uint2(start, start + leaf);
     if (c.start) c.start[idx] = start;
     if (c.skip) c.skip[idx] = skip;
+}
+
+template <int D>
+__device__ __forceinline__ void write_cell(const Cells &c, uint32_t idx, const Body &b, int level, double root_w,
+                                           uint32_t skip, uint32_t start, uint32_t leaf) {
+    const double inv = 1.0 / b.m;
+    const double cc[3] = {b.c0 * inv, b.c1 * inv, D == 3 ? b.c2 * inv : 0.0};
+    float hi[3], lo[3];
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        hi[a] = (float)cc[a];
+        lo[a] = (float)(cc[a] - (double)hi[a]);
+    }
+    put_cell<D>(c, idx, hi, lo, (float)b.m, level, root_w, skip, start, leaf);
+}
+
+// Leaf cell idx over the sorted points [a0, a1): of one point, the point itself,
+// exactly (no FP64 sums or quotient: most leaves, and FP64 was most of the
+// writer's time). parent_delta() gives the common bits of the leaf's parent, for
+// coincident points; alone: the tree is this one leaf.
+template <int D, typename PD>
+__device__ __forceinline__ void write_leaf(const Cells &c, uint32_t idx, const float4 *__restrict__ sp, uint32_t a0,
+                                           uint32_t a1, double root_w, bool alone, const PD &parent_delta) {
+    const float4 p = sp[a0];
+    if (a1 - a0 == 1) {
+        const float hi[3] = {p.x, p.y, p.z}, lo[3] = {0.f, 0.f, 0.f};
+        put_cell<D>(c, idx, hi, lo, p.w, alone ? 0 : parent_delta() / D + 1, root_w, idx + 1, a0, 1u);
+        return;
+    }
+    bool coinc;
+    const Body body = leaf_sum<D>(sp, a0, a1, coinc);
+    const int level = alone ? 0 : coinc ? parent_delta() / D + 1 : Levels<D>::L;
+    write_cell<D>(c, idx, body, level, root_w, idx + 1, a0, a1 - a0);
 }
 
 // Every cell at its preorder index, without walking chains: threads
@@ -1084,7 +1111,6 @@ __global__ void k_assign_cells(const DevState *st, BinTree t, uint32_t n_slots, 
                                DevState *stw) {
     gr_pdl_enter();
     if (st->converged) return;
-    constexpr int L = Levels<D>::L;
     const uint32_t nu = st->n_unique;
     const uint32_t ncells = st->n_cells;
     const double rw = st->root_w;
@@ -1098,12 +1124,7 @@ __global__ void k_assign_cells(const DevState *st, BinTree t, uint32_t n_slots, 
             atomicOr(&stw->error, (uint32_t)ERR_TREE);
             return;
         }
-        const float4 one = sp[a0];
-        bool coinc;
-        const Body body = leaf_sum<D>(sp, a0, a1, coinc);
-        // the parent's record only for coincident points (one leaf alone is the root)
-        const int level = nu == 1 ? 0 : coinc ? t.rec[t.leaf_parent[s]].w / D + 1 : L;
-        write_cell<D>(cells, idx, body, level, rw, idx + 1, a0, a1 - a0, a1 - a0 == 1 ? &one : nullptr);
+        write_leaf<D>(cells, idx, sp, a0, a1, rw, nu == 1, [&] { return t.rec[t.leaf_parent[s]].w; });
         leaf_pre[s] = idx;
         return;
     }

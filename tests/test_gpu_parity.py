@@ -348,6 +348,24 @@ def test_update_bounds_equal_the_bounds_pass(dim):
     assert ends[0][1] == ends[1][1]
 
 
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("lo,width", [(0.0, 0.5), (0.0, 1.0), (0.0, 3.9999998), (0.0, 4.0), (-0.5, 4.0), (-3.0, 8.0),
+                                      (-0.25, 1023.75), (-1000.0, 2047.9999), (-1000.0, 2048.0), (12.5, 1e6)])
+def test_the_root_square_at_the_edges_of_its_powers_of_two(dim, lo, width):
+    """Its doubling starts at half the widest side: the same square, so the same cells and interactions."""
+    n = 400
+    pos = np.random.default_rng(5).uniform(lo, lo + width, (n, dim)).astype(np.float32)
+    pos[0], pos[1] = lo, lo + width
+    src, dst = np.arange(n - 1, dtype=np.uint32), np.arange(1, n, dtype=np.uint32)
+    prm = dict(theta=0.9, dim=dim)
+    rel, info, _ = _check(n, src, dst, None, pos, prm)
+    st = oracle_state(n, src, dst, None, pos, prm)
+    st.accumulate(7)
+    assert info["n_cells"] == collapsed_cells(st)
+    far, pair = st.scalars()["far"], st.scalars()["pair"]
+    assert abs(info["far_count"] - far) <= 1e-3 * far + 2 and abs(info["pair_count"] - pair) <= 1e-3 * pair + 2
+
+
 def _full_sort_forces(n, src, dst, pos, prm):
     """Forces through gr_fa2_forces_static, which sorts the whole 64-bit key
     (8 passes) where a handle sorts the high word and fixes the runs."""
