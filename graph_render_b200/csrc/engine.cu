@@ -447,6 +447,71 @@ k_sort_small(const float4 *__restrict__ pos, uint32_t n, const DevState *st, uin
     }
 }
 
+// The smallest graphs: the keys and their sort without passes. A key's place in the
+// stable order is the number of keys below it and of equal ones before it: a block
+// owns RANK_KEYS keys, and its threads compute all n keys once more and count them
+// against each. What bounds it is that work, n^2 comparisons and n^2 / RANK_KEYS keys
+// over all SMs, so it ends where the blocks outnumber the SMs. A tick with it, with
+// k_sort_small and with the one-sweep passes, us: 300 nodes 46.8 / 50.4 / -, 1,500
+// 61.3 / 64.8 / 70.1; 3D 55.7 / 59.9 / 58.9, 74.7 / 78.2 / 87.1; a d3-force tick (two
+// sorts) 1,000 nodes 90.7 / 97.0, 2,000 101.8 / 111.6, 3,001 134.8 / 126.1. With 256
+// threads, or 32 keys a block, up to 4 us more.
+constexpr int RANK_T = 512, RANK_KEYS = 16;
+constexpr uint32_t RANK_MAX = 148 * RANK_KEYS;
+
+template <int D>
+__global__ void __launch_bounds__(RANK_T)
+k_rank_sort(const float4 *__restrict__ pos, uint32_t n, const DevState *st, uint64_t *__restrict__ keys_out,
+            uint32_t *__restrict__ vals_out) {
+    gr_pdl_enter();
+    if (st->converged) return;
+    __shared__ uint64_t s_key[RANK_KEYS];
+    __shared__ uint32_t s_below[RANK_T / GR_WARP][RANK_KEYS];
+    static_assert(RANK_T % RANK_KEYS == 0, "a block's keys lie in one slice");
+    const uint32_t t = threadIdx.x, i0 = blockIdx.x * RANK_KEYS;
+    const uint32_t own = i0 / RANK_T;  // the slice (RANK_T consecutive keys) of this block's keys
+    const double r0[3] = {st->root0[0], st->root0[1], D == 3 ? st->root0[2] : 0.0};
+    const double rw = st->root_w;
+    if (t < RANK_KEYS) s_key[t] = i0 + t < n ? morton_key<D>(pos[i0 + t], r0, rw) : ~0ull;
+    __syncthreads();
+    uint64_t key[RANK_KEYS];
+    uint32_t below[RANK_KEYS];
+#pragma unroll
+    for (int q = 0; q < RANK_KEYS; q++) {
+        key[q] = s_key[q];
+        below[q] = 0;
+    }
+    const uint32_t slices = (n + RANK_T - 1) / RANK_T;
+#pragma unroll 2
+    for (uint32_t r = 0; r < slices; r++) {
+        const uint32_t j = r * RANK_T + t;
+        const uint64_t k = j < n ? morton_key<D>(pos[j], r0, rw) : ~0ull;  // a key past the end is below none
+        if (r < own) {
+#pragma unroll
+            for (int q = 0; q < RANK_KEYS; q++) below[q] += k <= key[q] ? 1u : 0u;
+        } else if (r > own) {
+#pragma unroll
+            for (int q = 0; q < RANK_KEYS; q++) below[q] += k < key[q] ? 1u : 0u;
+        } else {
+#pragma unroll
+            for (int q = 0; q < RANK_KEYS; q++) below[q] += k < key[q] || (k == key[q] && j < i0 + q) ? 1u : 0u;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < RANK_KEYS; q++) {
+        const uint32_t b = __reduce_add_sync(GR_FULL, below[q]);
+        if (t % GR_WARP == 0) s_below[t / GR_WARP][q] = b;
+    }
+    __syncthreads();
+    if (t < RANK_KEYS && i0 + t < n) {
+        uint32_t at = 0;
+#pragma unroll
+        for (int w = 0; w < RANK_T / GR_WARP; w++) at += s_below[w][t];
+        keys_out[at] = s_key[t];
+        vals_out[at] = i0 + t;
+    }
+}
+
 // One-sweep passes of a tick's key sort for n nodes: the top 16 key bits up to
 // 2^14 nodes, 24 up to 2^22, else the high 32. The fewer the passes, the more
 // keys share their sorted bits and the longer the runs the fix-up puts in
@@ -460,11 +525,15 @@ static int sort_passes_for(uint32_t n) { return n <= (1u << 14) ? 2 : n <= (1u <
 // (k_fix_runs). The order is exactly the full stable 64-bit sort's. With an odd
 // pass count the keys are written to the sorter's scratch pair first, so the
 // last pass lands in keys/vals. The bounds pass zeroed os_ghist. Up to
-// SMALL_SORT_MAX nodes all of it is one kernel (k_sort_small).
+// SMALL_SORT_MAX nodes all of it is one kernel (k_rank_sort, k_sort_small).
 template <int D>
 static void keys_sort_fast(gr_fa2 *h, cudaStream_t s) {
     const uint32_t n = h->n;
     const uint32_t *conv = &h->st->converged;
+    if (n <= RANK_MAX) {
+        gr_launch(h->pdl, k_rank_sort<D>, div_up(n, RANK_KEYS), RANK_T, 0, s, h->pos, n, h->st, h->keys, h->vals);
+        return;
+    }
     if (n <= SMALL_SORT_MAX) {
         cudaFuncSetAttribute(k_sort_small<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMALL_SORT_SMEM);
         gr_launch(h->pdl, k_sort_small<D>, 1, SMALL_SORT_T, SMALL_SORT_SMEM, s, h->pos, n, h->st, h->keys, h->vals);

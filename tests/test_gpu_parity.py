@@ -447,6 +447,16 @@ def test_small_graph_sort_equals_the_full_sort(dim, n, cluster, spread):
 
 
 @pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("n", [2, 15, 16, 17, 511, 512, 513, 2367, 2368, 2369])
+@pytest.mark.parametrize("cluster,spread", [(0, 0.0), (1, 0.0), (9, 1e-3)])
+def test_rank_sort_equals_the_full_sort(dim, n, cluster, spread):
+    """Up to 2,368 nodes a key's place is counted (16 keys a block, 512 threads a slice), equal
+    keys in the order of their nodes: the full stable sort's order."""
+    pos, src, dst = _uniform_graph(n, dim, n + cluster + dim, min(cluster * n // 16, n), spread)
+    _fast_equals_full(n, dim, pos, src, dst)
+
+
+@pytest.mark.parametrize("dim", [2, 3])
 def test_engine_result_flows_through_the_snapshot_encoder(dim):
     """run_params (the registry face) -> Geometry -> the snapshot's binary face ->
     decode: the f32 columns come back bit for bit, in the topology's order."""
