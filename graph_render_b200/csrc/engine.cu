@@ -653,7 +653,17 @@ static void enqueue_tick(gr_fa2 *h, bool forces_only, int phases) {
             bt.delta = bt.int_parent = nullptr;
         }
         bt.marks = fold_scan ? h->scanner.bsum : nullptr;
-        gr_launch(h->pdl, k_karras<D>, gn, 256, 0, s, st, h->ukey, bt);
+        auto karras = [&](auto k, uint32_t threads, size_t smem) {
+            // one limit for every n: handles of several threads set it at once
+            if (smem > 48 * 1024)
+                cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)(KARRAS_STAGED_MAX * sizeof(uint64_t)));
+            gr_launch(h->pdl, k, div_up(n, threads), threads, smem, s, st, h->ukey, bt);
+        };
+        const int staged = karras_staged_threads(n);
+        if (staged == 256) karras(k_karras<D, 256>, 256, n * sizeof(uint64_t));
+        else if (staged == 512) karras(k_karras<D, 512>, 512, n * sizeof(uint64_t));
+        else karras(k_karras<D, 0>, 256, 0);
         if (adjoint) k_leaf_body<D><<<gn, 256, 0, s>>>(st, h->sp, h->leaf_start, h->leaf_body, h->leaf_coinc);
         if (adjoint) k_node_body<D><<<gn, 256, 0, s>>>(st, h->bt, pre, h->int_body);
         if (fold_scan)

@@ -349,6 +349,22 @@ def test_update_bounds_equal_the_bounds_pass(dim):
 
 
 @pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("n", [2, 257, 4096, 4097, 16384, 16385])
+def test_forces_either_side_of_the_staged_tree_build(n, dim):
+    """256 threads over keys in shared memory up to 4,096 nodes, 512 to 16,384, the keys in place past it;
+    a quarter of the points coincide, so there are fewer leaves than nodes."""
+    rng = np.random.default_rng(n)
+    pos = rng.uniform(-400, 400, (n, dim)).astype(np.float32)
+    pos[: n // 4] = pos[rng.integers(n // 4, n, n // 4)]
+    src, dst = np.arange(n - 1, dtype=np.uint32), np.arange(1, n, dtype=np.uint32)
+    prm = dict(theta=1.2, dim=dim, seed=2)
+    _, info, _ = _check(n, src, dst, None, pos, prm)
+    st = oracle_state(n, src, dst, None, pos, prm)
+    st.accumulate(7)
+    assert info["n_cells"] == collapsed_cells(st)
+
+
+@pytest.mark.parametrize("dim", [2, 3])
 @pytest.mark.parametrize("lo,width", [(0.0, 0.5), (0.0, 1.0), (0.0, 3.9999998), (0.0, 4.0), (-0.5, 4.0), (-3.0, 8.0),
                                       (-0.25, 1023.75), (-1000.0, 2047.9999), (-1000.0, 2048.0), (12.5, 1e6)])
 def test_the_root_square_at_the_edges_of_its_powers_of_two(dim, lo, width):
