@@ -12,6 +12,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <functional>
+#include <queue>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -1775,6 +1777,47 @@ static int batch_slots_for(int dim, int bt, bool wide, uint32_t *slots) {
     });
 }
 
+// The CTA size whose queue is estimated to end first. A CTA's tick of an n-node graph
+// takes a + b n us, fitted with every slot of the SMs taken (2D): small graphs want
+// many small CTAs, while one graph of 20,000 nodes outlasts the rest of a mixed batch
+// and wants all of an SM. The queue, largest first, is played over the slots; past 16
+// graphs a slot its length is the larger of the mean and the largest graph.
+// Two ticks with 256 / 512 / 1,024 threads, us: 512 graphs of 50 to 20,000 nodes 6546 /
+// 4511 / 2688, 2,048 of 50 to 2,000 781 / 909 / 1394, 2,048 of 1,500 2352 / 2244 / 2876,
+// 600 of 5,000 3666 / 3102 / 2920, 4,096 of 30 to 300 473 / 743 / 1714; of fourteen such
+// mixes the rule takes the fastest size in each.
+constexpr int BATCH_SIZES[3] = {256, 512, 1024};
+
+static int batch_pick_threads(const uint32_t *sorted_n, uint32_t graphs, const uint32_t *slots) {
+    const double a[3] = {8.4, 23.1, 24.8}, b[3] = {0.221, 0.1466, 0.053};
+    int pick = 0;
+    double best = INFINITY;
+    for (int i = 0; i < 3; i++) {
+        double end = 0.0;
+        if (graphs > 16 * slots[i]) {
+            for (uint32_t g = 0; g < graphs; g++) end += a[i] + b[i] * sorted_n[g];
+            end = std::max(end / slots[i], a[i] + b[i] * sorted_n[0]);
+        } else {
+            std::priority_queue<double, std::vector<double>, std::greater<double>> free_at;
+            for (uint32_t g = 0; g < graphs; g++) {
+                double t = 0.0;
+                if (free_at.size() == slots[i]) {
+                    t = free_at.top();
+                    free_at.pop();
+                }
+                t += a[i] + b[i] * sorted_n[g];
+                free_at.push(t);
+                end = std::max(end, t);
+            }
+        }
+        if (end < best) {
+            best = end;
+            pick = BATCH_SIZES[i];
+        }
+    }
+    return pick;
+}
+
 template <int D, int BT, bool WIDE>
 static int batch_launch(gr_fa2_batch *b, uint32_t ticks, uint32_t slots) {
     BatchArgs a;
@@ -1957,16 +2000,18 @@ int gr_fa2_batch_create(gr_fa2_batch **out, uint32_t ngraphs, const uint32_t *no
     for (uint32_t g = 0; g < ngraphs; g++) order[g] = g;
     std::stable_sort(order.begin(), order.end(),
                      [&](uint32_t a, uint32_t c) { return node_counts[a] > node_counts[c]; });
-    uint32_t slots = 0;
-    for (int bt : {256, 512, 1024}) {
-        uint32_t sl = 0;
-        if (int c = batch_slots_for(dim, bt, cells_wide(nmax), &sl)) {
+    uint32_t slots = 0, slots_of[3];
+    for (int i = 0; i < 3; i++) {
+        if (int c = batch_slots_for(dim, BATCH_SIZES[i], cells_wide(nmax), &slots_of[i])) {
             delete b;
             return c;
         }
-        slots = std::max(slots, sl);
+        slots = std::max(slots, slots_of[i]);
     }
     slots = std::min(slots, ngraphs);
+    std::vector<uint32_t> sorted_n(ngraphs);
+    for (uint32_t g = 0; g < ngraphs; g++) sorted_n[g] = node_counts[order[g]];
+    b->threads = batch_pick_threads(sorted_n.data(), ngraphs, slots_of);
     SlotView sv;
     b->slot_bytes = slot_carve(nullptr, nmax, dim, cells_wide(nmax), sv);
     b->max_slots = slots;
@@ -2018,7 +2063,7 @@ int gr_fa2_batch_tune(gr_fa2_batch *b, uint32_t sample_ticks, int *chosen, float
     CU(cudaMalloc(&save_s, sb));
     CU(cudaMemcpy(save_p, b->g->pos, pb, cudaMemcpyDeviceToDevice));
     CU(cudaMemcpy(save_s, b->d_state, sb, cudaMemcpyDeviceToDevice));
-    const int cands[3] = {256, 512, 1024};
+    const int *cands = BATCH_SIZES;
     float best = 1e30f;
     int pick = b->threads, rc = GR_OK;
     for (int i = 0; i < 3 && rc == GR_OK; i++) {

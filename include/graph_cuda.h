@@ -353,7 +353,8 @@ int gr_fa2_batch_create(gr_fa2_batch **out, uint32_t graphs, const uint32_t *nod
                         const double *weight, const double *params, uint32_t params_per_graph,
                         const float *pos0);
 void gr_fa2_batch_destroy(gr_fa2_batch *b);
-/* CTA size of the persistent kernel: 256, 512 (default) or 1024 threads. */
+/* CTA size of the persistent kernel: 256, 512 or 1024 threads (unless set, chosen by
+ * the graphs' sizes). */
 int gr_fa2_batch_set_threads(gr_fa2_batch *b, int threads);
 /* Autotuner: times sample_ticks ticks of the whole batch at each CTA size on a copy
  * of the state (restored afterwards) and keeps the fastest; ms_each (nullable, 3

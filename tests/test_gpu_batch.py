@@ -94,6 +94,23 @@ def test_graphs_either_side_of_the_block_sort_limit_match_the_engine():
         assert (int(st["far"][i]), int(st["pair"][i])) == (inf["far_count"], inf["pair_count"]), g.n
 
 
+@pytest.mark.parametrize("sizes", [[40] * 700 + [90], [700] * 460, [3000, 60, 60]], ids=["256", "512", "1024"])
+def test_threads_left_to_the_sizes_match_a_set_count(sizes, request):
+    """Mixes for which the queue is estimated to end first with 256, 512 and 1,024 threads: the result
+    of that count set by hand, bit for bit."""
+    gs = []
+    for i, n in enumerate(sizes):
+        rng = np.random.default_rng(i)
+        src, dst = rng.integers(0, n, (2, 2 * n)).astype(np.uint32)
+        pos = rng.uniform(0, 10 * n ** 0.5, (n, 2)).astype(np.float32)
+        gs.append(batch.GraphSpec(n, src, dst, dict(dim=2, theta=1.2, seed=i), None, pos, "random"))
+    with batch.Batch(gs) as b, batch.Batch(gs) as c:
+        c.set_threads(int(request.node.callspec.id))
+        b.run(1)
+        c.run(1)
+        assert all(np.array_equal(x, y) for x, y in zip(b.positions(), c.positions()))
+
+
 def test_first_tick_interactions_equal_the_one_graph_engine():
     gs = small_mix(16, seed=3)
     with batch.Batch(gs) as b:
