@@ -96,7 +96,7 @@ def walk_hbm_view(n: int, n_cells: int, dim: int, walk_ms: float) -> dict:
     """The walk against the measured HBM copy bandwidth: its algorithmic bytes per
     launch (every cell record and sorted node read once, the per-node indices read,
     the repulsion written) over the walk phase's time."""
-    cell_bytes = 32 if dim == 2 else 48
+    cell_bytes = 24 if dim == 2 else 32
     algo = n_cells * cell_bytes + n * (16 + 12) + n * dim * 4
     peak = None
     try:
@@ -107,7 +107,7 @@ def walk_hbm_view(n: int, n_cells: int, dim: int, walk_ms: float) -> dict:
     return {"bytes_per_launch": algo, "achieved": ach, "peak": peak, "unit": "GB/s",
             "frac": (ach / peak) if peak else None,
             "note": "cells x record size + nodes x (16 B point + 12 B indices) + nodes x dim x 4 B written; "
-                    "the walk is bound by instruction issue and load latency, not by this"}
+                    "the walk is bound by the L1's data pipe, not by this"}
 
 
 def workload(name: str, n: int = 0):
