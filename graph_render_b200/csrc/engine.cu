@@ -2401,7 +2401,7 @@ template <typename Offset>
 int bfs_levels(uint32_t n, const Offset *rp, const uint32_t *col, uint32_t k, const uint32_t *sources_dev,
                uint32_t *hops, DevBufs &B) {
     cudaStream_t s = B.s;
-    uint32_t *d_changed;  // [0]: the level before this round; [1 ..]: its own levels
+    uint32_t *d_changed;  // [0]: the level before these; [1 ..]: the levels launched together
     unsigned long long *vis, *fa, *fb;
     cudaError_t e;
     if ((e = B.get(&d_changed, BFS_AHEAD + 1)) || (e = B.get(&vis, n)) || (e = B.get(&fa, n)) || (e = B.get(&fb, n)))
